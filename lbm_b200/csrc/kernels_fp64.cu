@@ -410,7 +410,7 @@ poisson_init_kernel(Geom g, int h_loaded, const double* __restrict__ hload,
     const long long c = cell_of(g, x, y, z);
     const double pv = p[c];
     const double tauh = 1.0 / rho[c] + 0.5;
-    const double inv_tauh = 1.0 / tauh;
+    const RecipPair rt = recip_pair(tauh);
     const double sv = s[c];
     static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
@@ -420,8 +420,17 @@ poisson_init_kernel(Geom g, int h_loaded, const double* __restrict__ hload,
         const double h0 = source_aware ? E * pv - sa_scale * tauh * ((E / 3.0) * sv)
                                        : (h_loaded ? hload[(long long)q * g.n + c] : pv * E);
         const double hequ = E * pv;
-        hout[(long long)q * g.n + c] = h0 - div_rn(h0 - hequ, tauh, inv_tauh) - (E / 3.0) * sv;
+        hout[(long long)q * g.n + c] = h0 - div_rn(h0 - hequ, rt) - (E / 3.0) * sv;
     });
+}
+
+// Kinetic collision of one population, h - (h - E p) / tau - (E / 3) s
+// (CPU/Inamuro.cpp:755-778), the quotient from tau's reciprocal pair.
+template <int q>
+__device__ __forceinline__ double collide_h(double h, double pv, const RecipPair& rt, double sv)
+{
+    constexpr double E = wE(q);
+    return h - div_rn(h - E * pv, rt) - (E / 3.0) * sv;
 }
 
 // I: index type (long long in general, int where 15 n < 2^31).
@@ -429,15 +438,12 @@ template <class I>
 __device__ __forceinline__ void collide_h_store(const double (&hv)[Q], double pv, double tauh,
                                                 double sv, double* __restrict__ hout, I n, I c)
 {
-    const double inv_tauh = 1.0 / tauh;   // the 15 quotients by tau_h come from it (exact_div.cuh)
+    const RecipPair rt = recip_pair(tauh);   // the 15 quotients by tau_h come from it (exact_div.cuh)
     static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        constexpr double E = wE(q);
-        const double hequ = E * pv;
-        hout[(I)q * n + c] = hv[q] - div_rn(hv[q] - hequ, tauh, inv_tauh) - (E / 3.0) * sv;
+        hout[(I)q * n + c] = collide_h<q>(hv[q], pv, rt, sv);
     });
 }
-
 
 __device__ __forceinline__ double sum_q(const double (&hv)[Q])
 {
@@ -473,86 +479,122 @@ sweep_kernel(Geom g, const double* __restrict__ hin, double* __restrict__ hout,
     }
 }
 
-// Two sweeps in one pass (temporal blocking; same scheme as the mixed box).
-// A CTA owns a TX x TY xy tile and a run of `zlen` planes; marching in z it
-// computes sweep k on the tile plus a one-cell halo (wrapped coordinates,
-// pulled from global memory) into the z-grouped plane ring of lbm_device.cuh
-// (45 population planes), then sweep k+1 on the tile from that ring.  Every
-// cell's arithmetic is collide_h_store's expression, so (without FMA
-// contraction in this file) the result is bitwise that of two sweep_kernel
-// launches.  Each thread owns one halo-region cell for the whole march and
-// keeps the next plane's global pulls in flight while the CTA works through
-// the shared-memory phase; one barrier per plane.  lx % TX == 0,
-// ly % TY == 0 and 15 n < 2^31 are required (checked by the launcher).
-constexpr int F2_TX = 16, F2_TY = 8;
-constexpr int F2_RX = F2_TX + 2, F2_RY = F2_TY + 2, F2_RC = F2_RX * F2_RY;
-constexpr int F2_THREADS = (F2_RC + 31) / 32 * 32;   // 192: one thread per region cell
-constexpr int F2_SMEM = ring_planes() * F2_RC * (int)sizeof(double);   // 64,800 B
+// Two sweeps in one pass (temporal blocking): half the memory traffic of two
+// sweeps.  A CTA owns a 30 x 6 xy tile and marches a run of `zlen` planes in z;
+// each of its 256 threads owns one cell of the tile plus its one-cell halo (32
+// x 8, one warp per row) for the whole march.  Per plane it completes sweep k
+// at its cell of plane z+1 into a shared-memory plane ring, issues the pulls
+// of plane z+2 (in flight while the CTA works from the ring), and after a
+// barrier computes sweep k+1 of plane z at its own cell from the ring; a second
+// barrier frees the slots that the next plane overwrites, so population q
+// needs cz(q) + 2 slots (30 population planes).  tau_h's reciprocal pair and
+// the source of a cell are kept beside the ring for sweep k+1.  Coordinates
+// wrap, so the stream and the slip overwrite are those of two sweep_kernel
+// launches for any box, and every cell's arithmetic is collide_h's: the
+// result is bitwise theirs.  Cells outside the box (partial tiles) store
+// nothing.  15 n < 2^31 is required (the launcher checks).
+//
+// What bounds it: FP64 latency and the two barriers at 16 warps per SM; 126
+// registers (15 populations in flight and 15 at work) allow no more, and fewer
+// registers spill (0.54 ms per sweep at 96 registers, 0.62 at 80).  Measured on
+// B200 at 256^3, ms per sweep: 0.42 (5.1 TB/s of the 128 B/cell it moves)
+// against 0.65 for sweep_kernel; other shapes: 32 x 8 tiles with 11 warps in
+// one CTA 0.45, 30 x 14 in one CTA 0.47, 16 x 12 0.47; neighbouring warps
+// joined by named barriers in place of the CTA barriers 0.44; separate warps
+// for the two sweeps 0.47.
+constexpr int F2_RX = 32, F2_RY = 8;                     // region: tile and halo
+constexpr int F2_TX = F2_RX - 2, F2_TY = F2_RY - 2;      // tile
+constexpr int F2_RC = F2_RX * F2_RY;
+constexpr int F2_PLANES = 30;
+constexpr int F2_SMEM = (F2_PLANES + 2 * 3) * F2_RC * (int)sizeof(double);   // 73,728 B
 constexpr int F2_CTAS = 2;
 
-__global__ void __launch_bounds__(F2_THREADS, F2_CTAS)
+// Ring plane of population q of plane i (counted from the run's first halo plane).
+template <int q>
+__device__ __forceinline__ int f2_plane(int i)
+{
+    constexpr int slots = cz(q) + 2;
+    constexpr int base = cz(q) < 0 ? 0 : (cz(q) == 0 ? 5 : 15);
+    return base + (i % slots) * 5 + ring_rank(q);
+}
+
+__global__ void __launch_bounds__(F2_RC, F2_CTAS)
 sweep2_kernel(Geom g, int zlen, const double* __restrict__ hin, double* __restrict__ hout,
               const double* __restrict__ rho, const double* __restrict__ s)
 {
-    extern __shared__ double ring2[];   // [ring_planes()][F2_RC]
+    extern __shared__ double ring[];              // [F2_PLANES][F2_RC]
+    double* coef = ring + F2_PLANES * F2_RC;      // [2][3][F2_RC]: 1/tau_h (hi, lo), s
     const int t = threadIdx.x;
-    const int n = (int)g.n;
-    const int x0 = blockIdx.x * F2_TX, y0 = blockIdx.y * F2_TY;
+    const int lane = t % F2_RX, row = t / F2_RX;
+    const unsigned n = static_cast<unsigned>(g.n);
+    const unsigned plane = static_cast<unsigned>(g.lx) * g.ly;
     const int z0 = blockIdx.z * zlen;
     const int z1 = min(z0 + zlen, g.lz);
-    const bool owner = t < F2_RC;
-    const int xw = (x0 - 1 + t % F2_RX + g.lx) % g.lx;
-    const int yw = (y0 - 1 + t / F2_RX + g.ly) % g.ly;
+    const int x = blockIdx.x * F2_TX - 1 + lane, y = blockIdx.y * F2_TY - 1 + row;
+    const int xw = (x + g.lx) % g.lx, yw = (y + g.ly) % g.ly;
+    // in-plane parts of the pull offsets, indexed by 1 - c
+    const unsigned xs[3] = {static_cast<unsigned>(xw == 0 ? g.lx - 1 : xw - 1), static_cast<unsigned>(xw),
+                            static_cast<unsigned>(xw == g.lx - 1 ? 0 : xw + 1)};
+    const unsigned ys[3] = {static_cast<unsigned>(yw == 0 ? g.ly - 1 : yw - 1) * g.lx,
+                            static_cast<unsigned>(yw) * g.lx,
+                            static_cast<unsigned>(yw == g.ly - 1 ? 0 : yw + 1) * g.lx};
 
     double a[Q];
     double a_rho = 1.0, a_s = 0.0;
     auto prefetch = [&](int zz) {
-        if (!owner) return;
         const int zw = zz < 0 ? zz + g.lz : (zz >= g.lz ? zz - g.lz : zz);
-        pull_regs32(a, hin, n, g, xw, yw, zw);
-        const int c = (zw * g.ly + yw) * g.lx + xw;
+        const unsigned zs[3] = {(zw == 0 ? g.lz - 1 : zw - 1) * plane, zw * plane, (zw == g.lz - 1 ? 0 : zw + 1) * plane};
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            a[q] = __ldg(hin + (q * n + zs[1 - cz(q)]) + (ys[1 - cy(q)] + xs[1 - cx(q)]));
+        });
+        const unsigned c = zs[1] + ys[1] + xs[1];
         a_rho = __ldg(rho + c);
         a_s = __ldg(s + c);
     };
-    auto finish = [&](int zz) {
-        if (!owner) return;
+    auto finish = [&](int i) {
         bounce_regs(a, g, xw);
         const double pv = sum_q(a);
-        const double tauh = 1.0 / a_rho + 0.5;
-        // collide_h_store's expression, each population into its ring plane
-        const double inv_tauh = 1.0 / tauh;
+        const RecipPair rt = recip_pair(1.0 / a_rho + 0.5);
+        double* cf = coef + (i & 1) * 3 * F2_RC + t;
+        cf[0] = rt.hi;
+        cf[F2_RC] = rt.lo;
+        cf[2 * F2_RC] = a_s;
         static_for<0, Q>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
-            constexpr double E = wE(q);
-            const double hequ = E * pv;
-            ring2[ring_plane<q>(zz) * F2_RC + t] = a[q] - div_rn(a[q] - hequ, tauh, inv_tauh) - (E / 3.0) * a_s;
+            ring[f2_plane<q>(i) * F2_RC + t] = collide_h<q>(a[q], pv, rt, a_s);
         });
     };
 
     prefetch(z0 - 1);
-    finish(z0 - 1);
+    finish(0);
     prefetch(z0);
-    finish(z0);
+    finish(1);
     prefetch(z0 + 1);
-    const int tx = t % F2_TX, ty = t / F2_TX;
-    const int x = x0 + tx, y = y0 + ty;
-    const int rc = (ty + 1) * F2_RX + (tx + 1);
+    const bool inner = lane >= 1 && lane <= F2_TX && row >= 1 && row <= F2_TY && x < g.lx && y < g.ly;
     for (int z = z0; z < z1; ++z) {
-        finish(z + 1);
+        const int i = z - z0 + 1;
+        finish(i + 1);
         if (z + 1 < z1) prefetch(z + 2);
         __syncthreads();
-        if (t < F2_TX * F2_TY) {
+        if (inner) {
             double hv[Q];
             static_for<0, Q>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
-                hv[q] = ring2[ring_plane<q>(z - cz(q)) * F2_RC + rc - cy(q) * F2_RX - cx(q)];
+                hv[q] = ring[f2_plane<q>(i - cz(q)) * F2_RC + t - cy(q) * F2_RX - cx(q)];
             });
+            const double* cf = coef + (i & 1) * 3 * F2_RC + t;
+            const RecipPair rt{cf[0], cf[F2_RC]};
+            const double sv = cf[2 * F2_RC];
             bounce_regs(hv, g, x);
-            const int c = (z * g.ly + y) * g.lx + x;
+            const unsigned c = z * plane + ys[1] + xs[1];
             const double pv = sum_q(hv);
-            const double tauh = 1.0 / __ldg(rho + c) + 0.5;
-            collide_h_store(hv, pv, tauh, __ldg(s + c), hout, n, c);
+            static_for<0, Q>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                hout[q * n + c] = collide_h<q>(hv[q], pv, rt, sv);
+            });
         }
+        __syncthreads();
     }
 }
 
@@ -1142,19 +1184,33 @@ void sweep(cudaStream_t st, const Launch& L, const Geom& g, const double* hin, d
         sweep_kernel<false><<<L.grid, L.block, 0, st>>>(g, hin, hout, rho, s);
 }
 
-int sweep2_prepare(const Geom& g)
+bool sweep2_prepare(const Geom& g)
 {
-    if (g.lx % F2_TX != 0 || g.ly % F2_TY != 0 || g.lz < 3 || 15 * g.n >= 0x7fffffffLL) return 0;
-    if (cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F2_SMEM) != cudaSuccess)
-        return 0;
-    return 1;
+    return 15 * g.n < 0x7fffffffLL &&
+           cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F2_SMEM) == cudaSuccess;
+}
+
+// Two sweeps per pass where they are faster, from both sides' times on B200
+// (us per sweep): a pass takes 1.12 per wave and plane of its CTAs (128^3: 60
+// at 54, 256^3: 444 at 374, 96^3: 29 at 26, 64^3: 10.6 at 10), a single sweep
+// 39 per 10^6 cells from DRAM (128^3: 84, 72^3: 14.2, 90 x 75 x 131: 39) and
+// 2.2 + 21 per 10^6 cells while both h buffers stay in L2 (64^3: 7.8, 48^3:
+// 4.2, 32^3: 2.9; 240 B per cell, up to 3 * 10^5 cells).
+int sweep2_zlen(const Geom& g, int sms)
+{
+    const long long tiles = static_cast<long long>((g.lx + F2_TX - 1) / F2_TX) * ((g.ly + F2_TY - 1) / F2_TY);
+    long long cost = 0;
+    const int zlen = two_sweep_zlen(tiles, g.lz, F2_CTAS * sms, &cost);
+    const double mcells = 1e-6 * static_cast<double>(g.n);
+    const double single = mcells <= 0.3 ? 2.2 + 21.0 * mcells : 39.0 * mcells;
+    return 1.12 * static_cast<double>(cost) < single ? zlen : 0;
 }
 
 void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double* hout,
             const double* rho, const double* s)
 {
-    const dim3 grid(g.lx / F2_TX, g.ly / F2_TY, (g.lz + zlen - 1) / zlen);
-    sweep2_kernel<<<grid, F2_THREADS, F2_SMEM, st>>>(g, zlen, hin, hout, rho, s);
+    const dim3 grid((g.lx + F2_TX - 1) / F2_TX, (g.ly + F2_TY - 1) / F2_TY, (g.lz + zlen - 1) / zlen);
+    sweep2_kernel<<<grid, F2_RC, F2_SMEM, st>>>(g, zlen, hin, hout, rho, s);
 }
 
 void sweep_check_a(cudaStream_t st, const Launch& L, const Geom& g, const double* hin,

@@ -1200,10 +1200,10 @@ lbm_status lbm_create(const lbm_params* prm, lbm_precision precision, int device
     else st = mixed_alloc(h->mb, h->geom, h->L);
     if (st != LBM_OK) return bail(st);
     if (precision == LBM_PRECISION_FP64) {
-        // Two-sweep temporal blocking where the tile divides the box; the z
-        // run length can be tuned (0 disables) through LBM_SWEEP2_ZLEN.
+        // Two sweeps per pass where that is the faster form; LBM_SWEEP2_ZLEN
+        // sets the z run length (0: single sweeps).
         const char* env = std::getenv("LBM_SWEEP2_ZLEN");
-        const int zlen = env ? std::atoi(env) : 0;
+        const int zlen = env ? std::atoi(env) : fp64::sweep2_zlen(h->geom, prop.multiProcessorCount);
         h->fuse_zlen = (zlen > 0 && fp64::sweep2_prepare(h->geom)) ? zlen : 0;
         // z-marching collide where its tile divides the box (LBM_COLLIDE_ZLEN,
         // 0 disables).

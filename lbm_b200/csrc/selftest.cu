@@ -1,5 +1,5 @@
-// selftest.cu -- lbm_selftest_division: the FP64 kernels' correctly rounded
-// division from a reciprocal (exact_div.cuh) against CUDA's IEEE division on
+// selftest.cu -- lbm_selftest_division: the FP64 kernels' division from
+// a reciprocal pair (exact_div.cuh) against CUDA's IEEE division on
 // pseudo-random operands of the kinds the kernels use.
 #include <cuda_runtime.h>
 
@@ -45,8 +45,7 @@ __global__ void division_selftest_kernel(unsigned long long n, unsigned long lon
         case 4: b = random_double(r2, -10, 10, false); break;      // densities
         default: b = random_double(r2, -200, 200, true); break;   // any normal divisor
         }
-        const double y = 1.0 / b;
-        const double q = lbm::div_rn(a, b, y);
+        const double q = lbm::div_rn(a, lbm::recip_pair(b));
         const double ref = __ddiv_rn(a, b);
         if (__double_as_longlong(q) != __double_as_longlong(ref)) ++bad;
     }
