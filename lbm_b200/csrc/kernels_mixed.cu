@@ -187,7 +187,8 @@ sweep_kernel64(Geom g, const float* __restrict__ hin, float* __restrict__ hout,
 // one CTA per 32 x 8 tile of output cells and run of `zlen` planes; sweep k
 // on the tile plus its one-cell halo goes into a shared-memory plane ring,
 // sweep k+1 pulls from the ring and only the second result is written.
-// Requires lx % 32 == 0, ly % 8 == 0 and 15 n < 2^31 (the launcher checks).
+// Any box with 15 n < 2^31 (the launcher checks): tiles that reach past it
+// store nothing outside.
 constexpr int S2_TX = 32, S2_TY = 8;
 constexpr int S2_THREADS = sweep2_threads(S2_TX, S2_TY);   // 352: one thread per region cell
 constexpr int S2_SMEM = sweep2_smem(S2_TX, S2_TY);
@@ -468,6 +469,27 @@ float* field_f(MixedBuffers& mb, int which)
 
 }  // namespace
 
+namespace {
+
+// z run length of the two-sweep passes on any box (partial tiles store nothing
+// outside it), 0 where single sweeps are faster.  Both sides' times on B200
+// (us per sweep): a pass takes 0.95 per wave and plane of its CTAs (two per
+// SM; 128^3: 32 at 34, 256^3: 235 at 238, 64^3: 5.5 at 6), a single sweep 20.5
+// per 10^6 cells from DRAM (128^3: 45, 96^3: 18.5, 141 x 99 x 75: 27) and 1.75
+// + 13 per 10^6 cells while both h buffers stay in L2 (80^3: 8.5, 64^3: 4.9,
+// 32^3: 2.1; 120 B per cell, up to 7.5 * 10^5 cells).
+int sweep2_zlen(const Geom& g, int sms)
+{
+    const long long tiles = static_cast<long long>((g.lx + S2_TX - 1) / S2_TX) * ((g.ly + S2_TY - 1) / S2_TY);
+    long long cost = 0;
+    const int zlen = two_sweep_zlen(tiles, g.lz, 2LL * sms, &cost);
+    const double mcells = 1e-6 * static_cast<double>(g.n);
+    const double single = mcells <= 0.75 ? 1.75 + 13.0 * mcells : 20.5 * mcells;
+    return 0.95 * static_cast<double>(cost) < single ? zlen : 0;
+}
+
+}  // namespace
+
 lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
 {
     const size_t n = static_cast<size_t>(g.n);
@@ -487,32 +509,18 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
     }
     cudaMemset(mb.part_c, 0, 3 * nb * sizeof(double));
     mb.dwz = nullptr;
-    // Two-sweep temporal blocking where the tile divides the box, on z runs
-    // of the longest length in {32, 16, 8} whose grid still gives every SM
-    // 1.5 CTAs (shorter runs recompute more halo planes; a grid of fewer CTAs
-    // leaves SMs idle): measured on B200 (us per sweep, mixed), 128^3: 32.4
-    // at runs of 32 (256 CTAs); 96^3: 15.7 at 8 (432) against 22.2 at 32;
-    // 64^3 and 32^3: single sweeps 4.9 and 2.1 against 5.4 and 3.5 at the
-    // best run length, so no two-sweep pass below 1.5 CTAs per SM at runs of
-    // 8.  LBM_SWEEP2_ZLEN overrides (0 disables).
     mb.fuse_zlen = 0;
     int zlen = 0;
     if (const char* env = std::getenv("LBM_SWEEP2_ZLEN")) {
         zlen = std::atoi(env);
-    } else if (g.lx % S2_TX == 0 && g.ly % S2_TY == 0) {
+    } else {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             sms = 148;
-        const long long tiles = static_cast<long long>(g.lx / S2_TX) * (g.ly / S2_TY);
-        for (int zl : {32, 16, 8}) {
-            if (2 * tiles * ((g.lz + zl - 1) / zl) >= 3LL * sms) {
-                zlen = zl;
-                break;
-            }
-        }
+        zlen = sweep2_zlen(g, sms);
     }
-    if (zlen > 0 && g.lx % S2_TX == 0 && g.ly % S2_TY == 0 && g.lz >= 3 && 15 * g.n < 0x7fffffffLL &&
+    if (zlen > 0 && 15 * g.n < 0x7fffffffLL &&
         cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM) == cudaSuccess &&
         cudaFuncSetAttribute(sweep2_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM) ==
             cudaSuccess)
@@ -636,7 +644,7 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
     const float* omega = mb.dvy;
     int cur = start_parity;
     if (mb.fuse_zlen > 0) {
-        const dim3 grid(g.lx / S2_TX, g.ly / S2_TY, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
+        const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + S2_TY - 1) / S2_TY, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
         for (int i = 0; i + 1 < n_normal; i += 2) {
             sweep2_kernel<<<grid, S2_THREADS, S2_SMEM, st>>>(g, mb.fuse_zlen, mb.h[cur], mb.h[1 - cur],
                                                                      omega, mb.s);
@@ -718,7 +726,7 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
     int cur = 0;
     int i = 1;
     if (mb.fuse_zlen > 0) {
-        const dim3 grid(g.lx / S2_TX, g.ly / S2_TY, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
+        const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + S2_TY - 1) / S2_TY, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
         for (; i + 1 < n_normal; i += 2) {
             sweep2_refine_kernel<<<grid, S2_THREADS, S2_SMEM, st>>>(g, mb.fuse_zlen, e, mb.h[cur], omega, mb.rr);
             e = mb.h[cur];

@@ -25,7 +25,7 @@ def wavy_box(shape, periodic):
 
 # one tile with and without a remainder, several with one, extents below the
 # tile, one plane, z runs that do not divide the box
-@pytest.mark.parametrize("precision", ["fp64"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("shape,zlen", [((30, 6, 9), "4"), ((31, 7, 5), "5"), ((61, 13, 12), "5"), ((33, 9, 3), "2"),
                                         ((65, 17, 10), "32"), ((2, 1, 1), "1"), ((5, 40, 2), "8"), ((90, 3, 7), "3")])
 @pytest.mark.parametrize("periodic", [0, 1])
@@ -42,3 +42,19 @@ def test_two_sweep_pass_on_ragged_boxes(precision, shape, zlen, periodic, monkey
     assert got[0][1] == 0 and got[1][1] > 0
     for k in L.FIELDS:
         assert np.array_equal(got[0][0][k], got[1][0][k]), k
+
+
+@pytest.mark.parametrize("shape", [(45, 20, 14), (31, 9, 8)])
+def test_two_sweep_corrections_on_ragged_boxes(shape, monkeypatch):
+    p, f = wavy_box(shape, 0)
+    got = []
+    for z in ("0", "5"):
+        monkeypatch.setenv("LBM_SWEEP2_ZLEN", z)
+        g = L.InamuroCUDA(p, f, precision="mixed")
+        g.set_poisson(check_interval=20)
+        g.set_poisson_form("refine")
+        g.step_replay([40, 60])
+        got.append(g.download_fields())
+        g.close()
+    for k in L.FIELDS:
+        assert np.array_equal(got[0][k], got[1][k]), k
