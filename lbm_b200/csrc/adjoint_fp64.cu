@@ -421,36 +421,6 @@ padj_pi(Geom g, const double* __restrict__ y, double* __restrict__ pi)
     pi[c] = s;
 }
 
-// The transposed pull of all populations into (x, yy, z) (tpull's values): the
-// fifteen loads first, then the overwrite's transpose for the few columns it
-// concerns, so that no load waits for a branch (64^3: 12.4 -> 10.9 us a sweep).
-template <class I>
-__device__ __forceinline__ void tpull_all(double (&m)[Q], const double* __restrict__ y, I n, const Geom& g, const Wrap& w,
-                                          int x, int yy, int z)
-{
-    auto at = [&](auto kc, auto qc) {   // population k at the neighbour x + c_q
-        constexpr int k = decltype(kc)::value, q = decltype(qc)::value;
-        const I src = (static_cast<I>(pick<cz(q)>(w.zm, z, w.zp)) * static_cast<I>(g.ly) +
-                       static_cast<I>(pick<cy(q)>(w.ym, yy, w.yp))) * static_cast<I>(g.lx) +
-                      static_cast<I>(pick<cx(q)>(w.xm, x, w.xp));
-        return __ldg(y + static_cast<I>(k) * n + src);
-    };
-    static_for<0, Q>([&](auto qc) { m[decltype(qc)::value] = at(qc, qc); });
-    if (g.periodic_x) return;
-    if (w.xp == 0 || w.xp == g.lx - 1)
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            if constexpr (cx(q) == 1)
-                m[q] = w.xp == 0 ? 0.0 : m[q] + at(std::integral_constant<int, bounce_left(q)>{}, qc);
-        });
-    if (w.xm == g.lx - 1 || w.xm == 0)
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            if constexpr (cx(q) == -1)
-                m[q] = w.xm == g.lx - 1 ? 0.0 : m[q] + at(std::integral_constant<int, bounce_right(q)>{}, qc);
-        });
-}
-
 // One transposed sweep.  kCheck: also the relative change of
 // pi = sum_q y_q against the copy kept from the previous check (block
 // partials of sum |pi - pi_prev| and sum |pi|), and the new copy.  The pull

@@ -40,6 +40,7 @@
 #include "exact_div.cuh"
 #include "finalize.cuh"
 #include "lbm_solver.cuh"
+#include "sweep2_march.cuh"
 
 namespace lbm {
 namespace {
@@ -479,123 +480,35 @@ sweep_kernel(Geom g, const double* __restrict__ hin, double* __restrict__ hout,
     }
 }
 
-// Two sweeps in one pass (temporal blocking): half the memory traffic of two
-// sweeps.  A CTA owns a 30 x 6 xy tile and marches a run of `zlen` planes in z;
-// each of its 256 threads owns one cell of the tile plus its one-cell halo (32
-// x 8, one warp per row) for the whole march.  Per plane it completes sweep k
-// at its cell of plane z+1 into a shared-memory plane ring, issues the pulls
-// of plane z+2 (in flight while the CTA works from the ring), and after a
-// barrier computes sweep k+1 of plane z at its own cell from the ring; a second
-// barrier frees the slots that the next plane overwrites, so population q
-// needs cz(q) + 2 slots (30 population planes).  tau_h's reciprocal pair and
-// the source of a cell are kept beside the ring for sweep k+1.  Coordinates
-// wrap, so the stream and the slip overwrite are those of two sweep_kernel
-// launches for any box, and every cell's arithmetic is collide_h's: the
-// result is bitwise theirs.  Cells outside the box (partial tiles) store
-// nothing.  15 n < 2^31 is required (the launcher checks).
-//
-// What bounds it: FP64 latency and the two barriers at 16 warps per SM; 126
-// registers (15 populations in flight and 15 at work) allow no more, and fewer
-// registers spill (0.54 ms per sweep at 96 registers, 0.62 at 80).  Measured on
-// B200 at 256^3, ms per sweep: 0.42 (5.1 TB/s of the 128 B/cell it moves)
-// against 0.65 for sweep_kernel; other shapes: 32 x 8 tiles with 11 warps in
-// one CTA 0.45, 30 x 14 in one CTA 0.47, 16 x 12 0.47; neighbouring warps
-// joined by named barriers in place of the CTA barriers 0.44; separate warps
-// for the two sweeps 0.47.
-constexpr int F2_RX = 32, F2_RY = 8;                     // region: tile and halo
-constexpr int F2_TX = F2_RX - 2, F2_TY = F2_RY - 2;      // tile
-constexpr int F2_RC = F2_RX * F2_RY;
-constexpr int F2_PLANES = 30;
-constexpr int F2_SMEM = (F2_PLANES + 2 * 3) * F2_RC * (int)sizeof(double);   // 73,728 B
-constexpr int F2_CTAS = 2;
-
-// Ring plane of population q of plane i (counted from the run's first halo plane).
-template <int q>
-__device__ __forceinline__ int f2_plane(int i)
-{
-    constexpr int slots = cz(q) + 2;
-    constexpr int base = cz(q) < 0 ? 0 : (cz(q) == 0 ? 5 : 15);
-    return base + (i % slots) * 5 + ring_rank(q);
-}
+// Two sweeps in one pass (sweep2_march.cuh): every cell's arithmetic is
+// collide_h's, so the result is bitwise that of two sweep_kernel launches.
+struct SweepOps {
+    static constexpr int kCoefs = 3;   // tau_h's reciprocal pair, s
+    struct Fields {
+        double rho = 1.0, s = 0.0;
+    };
+    const double *rho, *s;
+    __device__ __forceinline__ Fields fields(unsigned c) const { return {__ldg(rho + c), __ldg(s + c)}; }
+    static __device__ __forceinline__ void cell(const Fields& f, double (&k)[3])
+    {
+        const RecipPair rt = recip_pair(1.0 / f.rho + 0.5);
+        k[0] = rt.hi;
+        k[1] = rt.lo;
+        k[2] = f.s;
+    }
+    template <int q>
+    static __device__ __forceinline__ double collide(double h, double pv, const double (&k)[3])
+    {
+        return collide_h<q>(h, pv, RecipPair{k[0], k[1]}, k[2]);
+    }
+};
 
 __global__ void __launch_bounds__(F2_RC, F2_CTAS)
 sweep2_kernel(Geom g, int zlen, const double* __restrict__ hin, double* __restrict__ hout,
               const double* __restrict__ rho, const double* __restrict__ s)
 {
-    extern __shared__ double ring[];              // [F2_PLANES][F2_RC]
-    double* coef = ring + F2_PLANES * F2_RC;      // [2][3][F2_RC]: 1/tau_h (hi, lo), s
-    const int t = threadIdx.x;
-    const int lane = t % F2_RX, row = t / F2_RX;
-    const unsigned n = static_cast<unsigned>(g.n);
-    const unsigned plane = static_cast<unsigned>(g.lx) * g.ly;
-    const int z0 = blockIdx.z * zlen;
-    const int z1 = min(z0 + zlen, g.lz);
-    const int x = blockIdx.x * F2_TX - 1 + lane, y = blockIdx.y * F2_TY - 1 + row;
-    const int xw = (x + g.lx) % g.lx, yw = (y + g.ly) % g.ly;
-    // in-plane parts of the pull offsets, indexed by 1 - c
-    const unsigned xs[3] = {static_cast<unsigned>(xw == 0 ? g.lx - 1 : xw - 1), static_cast<unsigned>(xw),
-                            static_cast<unsigned>(xw == g.lx - 1 ? 0 : xw + 1)};
-    const unsigned ys[3] = {static_cast<unsigned>(yw == 0 ? g.ly - 1 : yw - 1) * g.lx,
-                            static_cast<unsigned>(yw) * g.lx,
-                            static_cast<unsigned>(yw == g.ly - 1 ? 0 : yw + 1) * g.lx};
-
-    double a[Q];
-    double a_rho = 1.0, a_s = 0.0;
-    auto prefetch = [&](int zz) {
-        const int zw = zz < 0 ? zz + g.lz : (zz >= g.lz ? zz - g.lz : zz);
-        const unsigned zs[3] = {(zw == 0 ? g.lz - 1 : zw - 1) * plane, zw * plane, (zw == g.lz - 1 ? 0 : zw + 1) * plane};
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            a[q] = __ldg(hin + (q * n + zs[1 - cz(q)]) + (ys[1 - cy(q)] + xs[1 - cx(q)]));
-        });
-        const unsigned c = zs[1] + ys[1] + xs[1];
-        a_rho = __ldg(rho + c);
-        a_s = __ldg(s + c);
-    };
-    auto finish = [&](int i) {
-        bounce_regs(a, g, xw);
-        const double pv = sum_q(a);
-        const RecipPair rt = recip_pair(1.0 / a_rho + 0.5);
-        double* cf = coef + (i & 1) * 3 * F2_RC + t;
-        cf[0] = rt.hi;
-        cf[F2_RC] = rt.lo;
-        cf[2 * F2_RC] = a_s;
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            ring[f2_plane<q>(i) * F2_RC + t] = collide_h<q>(a[q], pv, rt, a_s);
-        });
-    };
-
-    prefetch(z0 - 1);
-    finish(0);
-    prefetch(z0);
-    finish(1);
-    prefetch(z0 + 1);
-    const bool inner = lane >= 1 && lane <= F2_TX && row >= 1 && row <= F2_TY && x < g.lx && y < g.ly;
-    for (int z = z0; z < z1; ++z) {
-        const int i = z - z0 + 1;
-        finish(i + 1);
-        if (z + 1 < z1) prefetch(z + 2);
-        __syncthreads();
-        if (inner) {
-            double hv[Q];
-            static_for<0, Q>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                hv[q] = ring[f2_plane<q>(i - cz(q)) * F2_RC + t - cy(q) * F2_RX - cx(q)];
-            });
-            const double* cf = coef + (i & 1) * 3 * F2_RC + t;
-            const RecipPair rt{cf[0], cf[F2_RC]};
-            const double sv = cf[2 * F2_RC];
-            bounce_regs(hv, g, x);
-            const unsigned c = z * plane + ys[1] + xs[1];
-            const double pv = sum_q(hv);
-            static_for<0, Q>([&](auto qc) {
-                constexpr int q = decltype(qc)::value;
-                hout[q * n + c] = collide_h<q>(hv[q], pv, rt, sv);
-            });
-        }
-        __syncthreads();
-    }
+    extern __shared__ double ring[];
+    sweep2_march(g, zlen, hin, hout, SweepOps{rho, s}, ring);
 }
 
 __global__ void __launch_bounds__(256)
@@ -1187,7 +1100,8 @@ void sweep(cudaStream_t st, const Launch& L, const Geom& g, const double* hin, d
 bool sweep2_prepare(const Geom& g)
 {
     return 15 * g.n < 0x7fffffffLL &&
-           cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F2_SMEM) == cudaSuccess;
+           cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                f2_smem(SweepOps::kCoefs)) == cudaSuccess;
 }
 
 // Two sweeps per pass where they are faster, from both sides' times on B200
@@ -1209,8 +1123,7 @@ int sweep2_zlen(const Geom& g, int sms)
 void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double* hout,
             const double* rho, const double* s)
 {
-    const dim3 grid((g.lx + F2_TX - 1) / F2_TX, (g.ly + F2_TY - 1) / F2_TY, (g.lz + zlen - 1) / zlen);
-    sweep2_kernel<<<grid, F2_RC, F2_SMEM, st>>>(g, zlen, hin, hout, rho, s);
+    sweep2_kernel<<<f2_grid(g, zlen), F2_RC, f2_smem(SweepOps::kCoefs), st>>>(g, zlen, hin, hout, rho, s);
 }
 
 void sweep_check_a(cudaStream_t st, const Launch& L, const Geom& g, const double* hin,

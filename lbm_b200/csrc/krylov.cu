@@ -17,10 +17,12 @@
 // added on the host.  The exit: ||b - (I - K) h||_2 < tolerance ||b||_2.
 #include <cuda_runtime.h>
 
+#include <cstdlib>
 #include <type_traits>
 
 #include "../../include/lbm_b200.h"
 #include "lbm_solver.cuh"
+#include "sweep2_march.cuh"
 
 namespace lbm {
 namespace {
@@ -49,7 +51,8 @@ __device__ __forceinline__ bool kcell(const Geom& g, int& x, int& y, int& z)
 // (the drift column), and sum_p asks for the partial sums of
 // sum_x (p(x) - p_ref), p = the sum of the pulled, bounced src, as one more
 // column (kinds 0-2: column 2; kind 3: column 0 of `part`).
-template <int kKind, bool kAdj>
+// I: the offset type (32-bit when 15 n < 2^31).
+template <int kKind, bool kAdj, class I>
 __global__ void __launch_bounds__(256)
 apply_kernel(Geom g, const double* __restrict__ in, const double* __restrict__ src, double* __restrict__ out,
              const double* __restrict__ rho, const double* __restrict__ s, const double* __restrict__ bvec,
@@ -60,18 +63,19 @@ apply_kernel(Geom g, const double* __restrict__ in, const double* __restrict__ s
     const bool active = kcell(g, x, y, z);
     double red[3] = {0.0, 0.0, 0.0};
     if (active) {
-        const long long n = g.n;
-        const long long c = cell_of(g, x, y, z);
+        const I n = static_cast<I>(g.n);
+        const I c = static_cast<I>(cell_of(g, x, y, z));
         const Wrap wr(g, x, y, z);
         double hv[Q];
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            if constexpr (kAdj)
-                hv[q] = tpull<q>(src, n, g, wr, x, y, z);
-            else
-                hv[q] = __ldg(src + (long long)q * n + pull_src<q>(g, wr, x, y, z));
-        });
-        if constexpr (!kAdj) bounce_regs(hv, g, x);
+        if constexpr (kAdj) {
+            tpull_all(hv, src, n, g, wr, x, y, z);
+        } else {
+            static_for<0, Q>([&](auto qc) {
+                constexpr int q = decltype(qc)::value;
+                hv[q] = __ldg(src + (static_cast<I>(q) * n + static_cast<I>(pull_src<q>(g, wr, x, y, z))));
+            });
+            bounce_regs(hv, g, x);
+        }
         double p = 0.0;
         static_for<0, Q>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
@@ -83,7 +87,7 @@ apply_kernel(Geom g, const double* __restrict__ in, const double* __restrict__ s
         static_for<0, Q>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
             constexpr double E = wE(q);
-            const long long i = (long long)q * n + c;
+            const I i = static_cast<I>(q) * n + c;
             const double kh = kAdj ? hv[q] - (hv[q] - p) * inv_tau : hv[q] - (hv[q] - E * p) * inv_tau;
             if constexpr (kKind == 3) {
                 out[i] = kh;
@@ -111,6 +115,37 @@ apply_kernel(Geom g, const double* __restrict__ in, const double* __restrict__ s
         double r2[2] = {red[0], red[1]};
         block_sum_store<2>(r2, part, nblocks, block_linear());
     }
+}
+
+template <int kKind, bool kAdj>
+auto apply_of(const Geom& g)
+{
+    return 15 * g.n < 0x7fffffffLL ? apply_kernel<kKind, kAdj, unsigned> : apply_kernel<kKind, kAdj, long long>;
+}
+
+// K twice in one pass (kind 3 twice; forward operator): half the memory traffic
+// of the applications between a polynomial's first and last.
+struct ApplyOps {
+    static constexpr int kCoefs = 1;   // 1 / tau_h
+    struct Fields {
+        double rho = 1.0;
+    };
+    const double* rho;
+    __device__ __forceinline__ Fields fields(unsigned c) const { return {__ldg(rho + c)}; }
+    static __device__ __forceinline__ void cell(const Fields& f, double (&k)[1]) { k[0] = 1.0 / (1.0 / f.rho + 0.5); }
+    template <int q>
+    static __device__ __forceinline__ double collide(double h, double p, const double (&k)[1])
+    {
+        constexpr double E = wE(q);
+        return h - (h - E * p) * k[0];
+    }
+};
+
+__global__ void __launch_bounds__(F2_RC, F2_CTAS)
+apply2_kernel(Geom g, int zlen, const double* __restrict__ in, double* __restrict__ out, const double* __restrict__ rho)
+{
+    extern __shared__ double ring[];
+    sweep2_march(g, zlen, in, out, ApplyOps{rho}, ring);
 }
 
 // Grid-stride vector updates over the 15 n populations.
@@ -189,6 +224,26 @@ shift_kernel(long long n, double* __restrict__ p, double* __restrict__ p_prev, d
 namespace krylov {
 namespace {
 
+// Where the applications between a polynomial's first (which sums p) and last
+// (which takes the inner products) run in pairs: the rule and the z runs of the
+// FP64 box's two-sweep passes, 0 elsewhere.  At 128^3 a pair takes 120 us, two
+// single applications 170 to 190; a degree-8 iteration 1.81 instead of 2.16 ms.
+// LBM_KRYLOV_PAIRS=0 turns them off.
+int pair_run(const Geom& g)
+{
+    const char* env = std::getenv("LBM_KRYLOV_PAIRS");
+    if (env && env[0] == '0') return 0;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    const int zlen = 15 * g.n < 0x7fffffffLL ? fp64::sweep2_zlen(g, sms) : 0;
+    return zlen > 0 && cudaFuncSetAttribute(apply2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            f2_smem(ApplyOps::kCoefs)) == cudaSuccess
+               ? zlen
+               : 0;
+}
+
 // BiCGSTAB iterations on (I - A_op) h = b from the initial guess in h; the
 // operator and source as apply_kernel<., kAdj>.  degree m > 1: the same
 // solution from the polynomially preconditioned system
@@ -216,6 +271,8 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
     const long long cnt = 15 * g.n;
     const int m = degree > 1 ? degree : 1;
     const bool border = !kAdj && !g.periodic_x;
+    // z run length of the pairs of applications (0: none), as the sweeps'
+    const int pair_zlen = !kAdj && m > 3 ? pair_run(g) : 0;
     double* psum_part = kb.part + 2 * L.nblocks;   // column 2 of the apply kernels' partial sums
     // out = in - A^m in (+ in_d E) (kinds 0, 2) or b_m - (in - A^m in + in_d E)
     // (kind 1), with the kind's partial sums; A^(m-1) in goes through
@@ -223,13 +280,19 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
     auto apply = [&](auto kindc, const double* in, double* out, const double* w, double in_d, double p_ref) {
         constexpr int kKind = decltype(kindc)::value;
         const double* src = in;
-        for (int j = 1; j < m; ++j) {
-            double* dst = (j & 1) ? kb.w1 : kb.w2;
-            apply_kernel<3, kAdj><<<L.grid, L.block, 0, st>>>(g, nullptr, src, dst, rho, nullptr, nullptr, nullptr,
-                                                               psum_part, L.nblocks, 0.0, border && j == 1, p_ref);
+        for (int j = 1; j < m;) {
+            double* dst = src == kb.w1 ? kb.w2 : kb.w1;
+            if (j > 1 && j + 1 < m && pair_zlen > 0) {
+                apply2_kernel<<<f2_grid(g, pair_zlen), F2_RC, f2_smem(ApplyOps::kCoefs), st>>>(g, pair_zlen, src, dst, rho);
+                j += 2;
+            } else {
+                apply_of<3, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, nullptr, src, dst, rho, nullptr, nullptr, nullptr,
+                                                                   psum_part, L.nblocks, 0.0, border && j == 1, p_ref);
+                ++j;
+            }
             src = dst;
         }
-        apply_kernel<kKind, kAdj><<<L.grid, L.block, 0, st>>>(g, in, src, out, rho, s, m > 1 ? kb.bm : nullptr, w,
+        apply_of<kKind, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, in, src, out, rho, s, m > 1 ? kb.bm : nullptr, w,
                                                               kb.part, L.nblocks, border ? in_d : 0.0,
                                                               border && m == 1, p_ref);
     };
@@ -255,14 +318,14 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
     if (cudaMemsetAsync(kb.v, 0, static_cast<size_t>(cnt) * sizeof(double), st) != cudaSuccess) return LBM_ERR_CUDA;
     if (m > 1) {
         // b_m = b + A b + ... + A^(m-1) b (b: the kind-1 residual of x = 0)
-        apply_kernel<1, kAdj><<<L.grid, L.block, 0, st>>>(g, kb.v, kb.v, kb.bm, rho, s, nullptr, nullptr, kb.part,
+        apply_of<1, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, kb.v, kb.v, kb.bm, rho, s, nullptr, nullptr, kb.part,
                                                           L.nblocks, 0.0, 0, 0.0);
         vec_kernel<3><<<kDotBlocks, 256, 0, st>>>(cnt, 0.0, 0.0, kb.w1, kb.w2, kb.bm, nullptr, nullptr, nullptr,
                                                    nullptr);
         const double* cur = kb.w1;
         for (int j = 1; j < m; ++j) {
             double* dst = (j & 1) ? kb.w2 : kb.w1;
-            apply_kernel<3, kAdj><<<L.grid, L.block, 0, st>>>(g, nullptr, cur, dst, rho, nullptr, nullptr, nullptr,
+            apply_of<3, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, nullptr, cur, dst, rho, nullptr, nullptr, nullptr,
                                                                nullptr, 0, 0.0, 0, 0.0);
             vec_kernel<4><<<kDotBlocks, 256, 0, st>>>(cnt, 0.0, 0.0, kb.bm, nullptr, dst, nullptr, nullptr, nullptr,
                                                        nullptr);
