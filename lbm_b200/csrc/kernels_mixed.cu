@@ -179,39 +179,46 @@ sweep_kernel64(Geom g, const float* __restrict__ hin, float* __restrict__ hout,
     float hv[Q];
     pull_regs(hv, hin, g, x, y, z);
     bounce_regs(hv, g, x);
-    const P32 ps = sum_q32(hv);
+    const P32Hi ps = sum_q32(hv);
     collide_h_store(hv, (double)ps.hi + (double)ps.lo, __ldg(omega + c), __ldg(s + c), hout, g.n, c);
 }
 
 // Two sweeps in one pass (temporal blocking, sweep2_run in mixed_cells.cuh):
-// one CTA per 32 x 8 tile of output cells and run of `zlen` planes; sweep k
-// on the tile plus its one-cell halo goes into a shared-memory plane ring,
-// sweep k+1 pulls from the ring and only the second result is written.
+// one CTA per 32 x 8 or 32 x 16 tile of output cells and run of `zlen` planes;
+// sweep k on the tile plus its one-cell halo goes into a shared-memory plane
+// ring, sweep k+1 pulls from the ring and only the second result is written.
 // Any box with 15 n < 2^31 (the launcher checks): tiles that reach past it
-// store nothing outside.
+// store nothing outside.  Bound by instruction issue and load latency at 22 or
+// 20 warps per SM (33 M warp instructions per launch at 128^3, 55 % issue,
+// 0.75 of the HBM rate).  Measured at 256^3 (B200), ms per sweep: 0.222 on 32 x
+// 16 tiles, 0.226 on 32 x 8, 0.235 with one barrier and 45 ring planes; TMA
+// loads of the tiles 0.28 (230 cycles per ten-row box), two cells per thread in
+// packed FP32 pairs 0.235 to 0.28 (as many instructions, fewer warps).
 constexpr int S2_TX = 32, S2_TY = 8;
-constexpr int S2_THREADS = sweep2_threads(S2_TX, S2_TY);   // 352: one thread per region cell
-constexpr int S2_SMEM = sweep2_smem(S2_TX, S2_TY);
+constexpr int S2_TALL = 16;   // the tall tile: 640 threads in one CTA per SM, 83 KB (32 x 8: 352 in two, 46 KB each)
 
-__global__ void __launch_bounds__(S2_THREADS, 2)
+template <int TY, int kCtas>
+__global__ void __launch_bounds__(sweep2_threads(S2_TX, TY), kCtas)
 sweep2_kernel(Geom g, int zlen, const float* __restrict__ hin, float* __restrict__ hout,
               const float* __restrict__ omega, const float* __restrict__ s)
 {
     extern __shared__ float ring[];
     const int z0 = blockIdx.z * zlen;
-    sweep2_run<S2_TX, S2_TY>(g, blockIdx.x * S2_TX, blockIdx.y * S2_TY, z0, min(z0 + zlen, g.lz), hin, hout, omega,
-                             s, ring);
+    sweep2_run<S2_TX, TY>(g, blockIdx.x * S2_TX, blockIdx.y * TY, z0, min(z0 + zlen, g.lz), hin, hout, omega, s, ring);
 }
 
-// The refinement form's correction sweeps two per pass (sweep2_run<., ., true>).
-__global__ void __maxnreg__(88)
+// The refinement form's correction sweeps two per pass (sweep2_run<., ., true>),
+// on the tall tile: the source r takes 15 registers more, at which one CTA of
+// the 32 x 8 tile's 11 warps is all an SM holds (128^3: 62.5 -> 59.4 us per
+// sweep of a check interval, 256^3: 456 -> 436, 90 x 75 x 131: 28.8 -> 28.0).
+__global__ void __launch_bounds__(sweep2_threads(S2_TX, S2_TALL), 1)
 sweep2_refine_kernel(Geom g, int zlen, const float* __restrict__ ein, float* __restrict__ eout,
                      const float* __restrict__ omega, const float* __restrict__ r)
 {
     extern __shared__ float ring[];
     const int z0 = blockIdx.z * zlen;
-    sweep2_run<S2_TX, S2_TY, true>(g, blockIdx.x * S2_TX, blockIdx.y * S2_TY, z0, min(z0 + zlen, g.lz), ein, eout,
-                                   omega, r, ring);
+    sweep2_run<S2_TX, S2_TALL, true>(g, blockIdx.x * S2_TX, blockIdx.y * S2_TALL, z0, min(z0 + zlen, g.lz), ein, eout,
+                                     omega, r, ring);
 }
 
 __global__ void __launch_bounds__(256)
@@ -472,20 +479,27 @@ float* field_f(MixedBuffers& mb, int which)
 namespace {
 
 // z run length of the two-sweep passes on any box (partial tiles store nothing
-// outside it), 0 where single sweeps are faster.  Both sides' times on B200
-// (us per sweep): a pass takes 0.95 per wave and plane of its CTAs (two per
-// SM; 128^3: 32 at 34, 256^3: 235 at 238, 64^3: 5.5 at 6), a single sweep 20.5
-// per 10^6 cells from DRAM (128^3: 45, 96^3: 18.5, 141 x 99 x 75: 27) and 1.75
-// + 13 per 10^6 cells while both h buffers stay in L2 (80^3: 8.5, 64^3: 4.9,
-// 32^3: 2.1; 120 B per cell, up to 7.5 * 10^5 cells).
-int sweep2_zlen(const Geom& g, int sms)
+// outside it) and whether they take the tall tile; 0 where single sweeps are
+// faster (*zlen_tall: the tall tile's in any case).  Both sides' times on B200 (us per sweep): a pass takes 0.93 per wave
+// and plane of its CTAs on 32 x 8 tiles (two per SM; 128^3: 29.8 at 34, 256^3:
+// 226 at 238, 141 x 99 x 141: 31.9 at 36) and 0.91 on 32 x 16 (one per SM; 29.1,
+// 223, 34.2 at 38), a single sweep 20.5 per 10^6 cells from DRAM (128^3: 45,
+// 96^3: 18.5, 141 x 99 x 75: 27) and 1.75 + 13 per 10^6 cells while both h
+// buffers stay in L2 (80^3: 8.5, 64^3: 4.9, 32^3: 2.1; 120 B per cell, up to
+// 7.5 * 10^5 cells).
+int sweep2_zlen(const Geom& g, int sms, bool* tall, int* zlen_tall)
 {
-    const long long tiles = static_cast<long long>((g.lx + S2_TX - 1) / S2_TX) * ((g.ly + S2_TY - 1) / S2_TY);
-    long long cost = 0;
-    const int zlen = two_sweep_zlen(tiles, g.lz, 2LL * sms, &cost);
+    auto tiles = [&](int ty) {
+        return static_cast<long long>((g.lx + S2_TX - 1) / S2_TX) * ((g.ly + ty - 1) / ty);
+    };
+    long long low_cost = 0, tall_cost = 0;
+    const int low = two_sweep_zlen(tiles(S2_TY), g.lz, 2LL * sms, &low_cost);
+    const int high = *zlen_tall = two_sweep_zlen(tiles(S2_TALL), g.lz, sms, &tall_cost);
+    *tall = tall_cost <= low_cost;
     const double mcells = 1e-6 * static_cast<double>(g.n);
     const double single = mcells <= 0.75 ? 1.75 + 13.0 * mcells : 20.5 * mcells;
-    return 0.95 * static_cast<double>(cost) < single ? zlen : 0;
+    const double pass = *tall ? 0.91 * static_cast<double>(tall_cost) : 0.93 * static_cast<double>(low_cost);
+    return pass < single ? (*tall ? high : low) : 0;
 }
 
 }  // namespace
@@ -510,21 +524,25 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
     cudaMemset(mb.part_c, 0, 3 * nb * sizeof(double));
     mb.dwz = nullptr;
     mb.fuse_zlen = 0;
-    int zlen = 0;
+    mb.fuse_tall = false;
+    int zlen = 0, zlen_tall = 0;
     if (const char* env = std::getenv("LBM_SWEEP2_ZLEN")) {
-        zlen = std::atoi(env);
+        zlen = zlen_tall = std::atoi(env);
     } else {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             sms = 148;
-        zlen = sweep2_zlen(g, sms);
+        zlen = sweep2_zlen(g, sms, &mb.fuse_tall, &zlen_tall);
     }
     if (zlen > 0 && 15 * g.n < 0x7fffffffLL &&
-        cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM) == cudaSuccess &&
-        cudaFuncSetAttribute(sweep2_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S2_SMEM) ==
-            cudaSuccess)
+        cudaFuncSetAttribute(sweep2_kernel<S2_TALL, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess &&
+        cudaFuncSetAttribute(sweep2_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess) {
         mb.fuse_zlen = zlen;
+        mb.refine_zlen = zlen_tall;
+    }
     // z-marching collide where its tile divides the box.
     const char* cenv = std::getenv("LBM_COLLIDE_ZLEN");
     const int czlen = cenv ? std::atoi(cenv) : 16;
@@ -644,10 +662,12 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
     const float* omega = mb.dvy;
     int cur = start_parity;
     if (mb.fuse_zlen > 0) {
-        const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + S2_TY - 1) / S2_TY, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
+        const int ty = mb.fuse_tall ? S2_TALL : S2_TY;
+        const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + ty - 1) / ty, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
+        auto kern = mb.fuse_tall ? sweep2_kernel<S2_TALL, 1> : sweep2_kernel<S2_TY, 2>;
         for (int i = 0; i + 1 < n_normal; i += 2) {
-            sweep2_kernel<<<grid, S2_THREADS, S2_SMEM, st>>>(g, mb.fuse_zlen, mb.h[cur], mb.h[1 - cur],
-                                                                     omega, mb.s);
+            kern<<<grid, sweep2_threads(S2_TX, ty), sweep2_smem(S2_TX, ty), st>>>(g, mb.fuse_zlen, mb.h[cur], mb.h[1 - cur],
+                                                                                  omega, mb.s);
             cur = 1 - cur;
         }
         n_normal &= 1;
@@ -726,9 +746,11 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
     int cur = 0;
     int i = 1;
     if (mb.fuse_zlen > 0) {
-        const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + S2_TY - 1) / S2_TY, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
+        const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + S2_TALL - 1) / S2_TALL,
+                        (g.lz + mb.refine_zlen - 1) / mb.refine_zlen);
         for (; i + 1 < n_normal; i += 2) {
-            sweep2_refine_kernel<<<grid, S2_THREADS, S2_SMEM, st>>>(g, mb.fuse_zlen, e, mb.h[cur], omega, mb.rr);
+            sweep2_refine_kernel<<<grid, sweep2_threads(S2_TX, S2_TALL), sweep2_smem(S2_TX, S2_TALL), st>>>(
+                g, mb.refine_zlen, e, mb.h[cur], omega, mb.rr);
             e = mb.h[cur];
             cur = 1 - cur;
         }

@@ -193,16 +193,14 @@ __device__ __forceinline__ void pull_regs32(T (&v)[Q], const T* __restrict__ src
 
 // ---- plane ring of the two-sweep passes --------------------------------
 // A two-sweep pass marches a tile in z: at iteration z it writes sweep k's
-// populations of plane z+1 into a shared-memory ring (before the iteration's
-// barrier) and, after the barrier, pulls sweep k+1's populations of plane z
-// from it -- population q from plane z - cz(q).  So plane P's population q is
-// read at iteration P-1 (cz = -1), P (cz = 0) or P+1 (cz = +1), and a slot may
-// be rewritten only after every thread has passed the barrier that follows
-// its last read: the three groups of five populations (by cz) need 2, 3 and 4
-// plane slots, 45 population planes in all (4 x 15 without the grouping).
-__host__ __device__ constexpr int ring_group_slots(int g) { return g + 2; }   // g = cz + 1
-__host__ __device__ constexpr int ring_group_base(int g) { return g == 0 ? 0 : (g == 1 ? 10 : 25); }
-__host__ __device__ constexpr int ring_planes() { return 45; }   // population planes
+// populations of plane z+1 into a shared-memory ring and, after a barrier, pulls
+// sweep k+1's populations of plane z from it -- population q from plane z -
+// cz(q); a second barrier ends the iteration.  So plane P's population q is
+// written at iteration P-1 and last read at iteration P + cz(q), and the three
+// groups of five populations (by cz) need 1, 2 and 3 plane slots: 30 population
+// planes.  (With one barrier per iteration a slot more each, 45 planes: the
+// shared memory that takes from L1 costs more than the barrier.)
+__host__ __device__ constexpr int ring_planes() { return 30; }
 // Rank of q among the populations with the same cz.
 __host__ __device__ constexpr int ring_rank(int q)
 {
@@ -210,14 +208,13 @@ __host__ __device__ constexpr int ring_rank(int q)
     for (int k = 0; k < q; ++k) r += (cz(k) == cz(q)) ? 1 : 0;
     return r;
 }
-// Population plane of (q, plane zz) in the ring.
+// Population plane of q's plane i >= 0 (counted from the run's first halo plane).
 template <int q>
-__device__ __forceinline__ int ring_plane(int zz)
+__device__ __forceinline__ int ring_plane(int i)
 {
-    constexpr int gq = cz(q) + 1;
-    constexpr int S = ring_group_slots(gq);
-    const int slot = ((zz % S) + S) % S;
-    return ring_group_base(gq) + slot * 5 + ring_rank(q);
+    constexpr int slots = cz(q) + 2;
+    constexpr int base = cz(q) < 0 ? 0 : (cz(q) == 0 ? 5 : 15);
+    return base + (i % slots) * 5 + ring_rank(q);
 }
 
 // x slip overwrite of pulled populations (CPU/Inamuro.cpp:589-623).

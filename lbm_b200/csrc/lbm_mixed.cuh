@@ -28,6 +28,8 @@ struct MixedBuffers {
     double* hd[2] = {nullptr, nullptr};
     float* rr = nullptr;
     int fuse_zlen = 0;           // >0: plain sweeps run two per pass, z runs of this length
+    bool fuse_tall = false;      // ... on 32 x 16 tiles instead of 32 x 8
+    int refine_zlen = 0;         // z runs of the correction sweeps' passes (with fuse_zlen)
     int collide_zlen = 0;        // >0: z-marching collide, z runs of this length
     bool allocated = false;
 };

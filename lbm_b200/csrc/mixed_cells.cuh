@@ -133,6 +133,12 @@ __device__ __forceinline__ float mix_div(const CellDeriv<float>& d, double (&red
 struct P32 {
     float hi, lo;
 };
+// One with lo = 0 (the plain sweeps' FP32 sum): collide_h leaves out lo's FMA,
+// which would add -0.
+struct P32Hi {
+    float hi;
+    static constexpr float lo = 0.f;
+};
 __device__ __forceinline__ P32 p32_of(double pv)
 {
     P32 r;
@@ -153,14 +159,14 @@ __device__ __forceinline__ P32 p32_of(double pv)
 // is formed from the small terms alone, and h gains it in one rounding, so a
 // population at its fixed point stays there.  (Measured at 256^3 against the
 // FP64 box, 3 steps x 1000 sweeps: p error 2.2e-5 with the plain expression.)
-template <int q>
-__device__ __forceinline__ float collide_h(float h, P32 p, float om, float sv)
+template <int q, class P>
+__device__ __forceinline__ float collide_h(float h, P p, float om, float sv)
 {
     constexpr float E = float(wE(q));
     constexpr float El = float(wE(q) - double(float(wE(q))));   // E = E + El to FP64 precision
     constexpr float E3 = float(wE(q) / 3.0);
     float t = fmaf(-E, p.hi, h);
-    t = fmaf(-E, p.lo, t);
+    if constexpr (!std::is_same<P, P32Hi>::value) t = fmaf(-E, p.lo, t);
     t = fmaf(-El, p.hi, t);
     return h + fmaf(-om, t, -(E3 * sv));
 }
@@ -183,38 +189,13 @@ __device__ __forceinline__ double sum_q(const float (&hv)[Q])
 }
 
 // p = sum_q h of the plain sweeps (the check kernels sum in FP64).
-#ifndef LBM_PSUM
-#define LBM_PSUM 0
-#endif
-__device__ __forceinline__ P32 sum_q32(const float (&h)[Q])
+__device__ __forceinline__ P32Hi sum_q32(const float (&h)[Q])
 {
-#if LBM_PSUM == 0
-    P32 r;
-    r.lo = 0.f;
-    r.hi = (((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]))) +
-           (((h[8] + h[9]) + (h[10] + h[11])) + ((h[12] + h[13]) + h[14]));
-    return r;
-#elif LBM_PSUM == 1
-    double acc = 0.0;
-    static_for<0, Q>([&](auto qc) { acc += (double)h[decltype(qc)::value]; });
-    return p32_of(acc);
-#else
-    float s = h[0], c = 0.f;
-    static_for<1, Q>([&](auto qc) {
-        const float x = h[decltype(qc)::value];
-        const float tt = s + x;
-        const float z = tt - s;
-        c += (s - (tt - z)) + (x - z);
-        s = tt;
-    });
-    P32 r;
-    r.hi = s + c;
-    r.lo = c - (r.hi - s);
-    return r;
-#endif
+    return {(((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]))) +
+            (((h[8] + h[9]) + (h[10] + h[11])) + ((h[12] + h[13]) + h[14]))};
 }
 
-__device__ __forceinline__ void collide_h_store32(const float (&hv)[Q], P32 p32, float om, float sv,
+__device__ __forceinline__ void collide_h_store32(const float (&hv)[Q], P32Hi p32, float om, float sv,
                                                   float* __restrict__ hout, int n, int c)
 {
     static_for<0, Q>([&](auto qc) {
@@ -464,23 +445,23 @@ __device__ __forceinline__ void mixc_correct(const Geom& g, float* __restrict__ 
 }
 
 // Two kinetic sweeps of the z run [z0, z1) of the TX x TY column at (x0, y0)
-// (temporal blocking; the single box's sweep2_kernel and the batched
+// (temporal blocking; the single box's sweep2_kernels and the batched
 // b_sweep2 run this body).  Threads: one per cell of the tile plus its
 // one-cell halo, (TX+2)(TY+2) rounded up to whole warps.  Each thread owns one
 // region cell for the whole march and keeps the global pulls of the NEXT
 // plane in flight (registers) while the CTA works through the shared-memory
-// phase of the current one; one barrier per plane.  Region cells use wrapped
+// phase of the current one; two barriers per plane.  Region cells use wrapped
 // coordinates, so the periodic stream and the x slip overwrite are those of
 // two single sweeps; tile cells outside the box (partial tiles) store
-// nothing.  Cell arithmetic: mixc_sweep32's (collide_h, sum_q32).  The ring
-// is the z-direction-grouped one of lbm_device.cuh (ring_plane, 45 population
-// planes).  kRefine: the refinement form's correction sweeps instead,
-// e' = K e + r with r a per-population source (src = r, 15 n floats), the
-// arithmetic of refine_sweep_kernel.
+// nothing.  Cell arithmetic: mixc_sweep32's (collide_h, sum_q32), so bitwise
+// its result.  The ring is that of lbm_device.cuh (30 population planes), with
+// the cells' omega and s kept beside it for sweep k+1.  kRefine: the refinement
+// form's correction sweeps instead, e' = K e + r with r a per-population source
+// (src = r, 15 n floats), the arithmetic of refine_sweep_kernel.
 __host__ __device__ constexpr int sweep2_threads(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32 * 32; }
 __host__ __device__ constexpr int sweep2_smem(int tx, int ty)
 {
-    return ring_planes() * (tx + 2) * (ty + 2) * static_cast<int>(sizeof(float));
+    return (ring_planes() + 2 * 2) * (tx + 2) * (ty + 2) * static_cast<int>(sizeof(float));
 }
 
 // Correction-sweep update of the refinement form: K e + r in FP32.
@@ -503,12 +484,20 @@ __device__ __forceinline__ void sweep2_run(const Geom& g, int x0, int y0, int z0
                                            float* __restrict__ ring)
 {
     constexpr int RX = TX + 2, RC = RX * (TY + 2);
+    float* coef = ring + ring_planes() * RC;   // [2][2][RC]: omega, s
     const int t = threadIdx.x;
-    const int n = (int)g.n;
-    // this thread's halo-region cell (wrapped coordinates)
+    const unsigned n = static_cast<unsigned>(g.n);
+    const unsigned plane = static_cast<unsigned>(g.lx) * g.ly;
+    // this thread's halo-region cell (wrapped coordinates) and the in-plane
+    // parts of its pull offsets, indexed by 1 - c
     const bool owner = t < RC;
     const int xw = (x0 - 1 + t % RX + g.lx) % g.lx;
     const int yw = (y0 - 1 + t / RX + g.ly) % g.ly;
+    const unsigned xs[3] = {static_cast<unsigned>(xw == 0 ? g.lx - 1 : xw - 1), static_cast<unsigned>(xw),
+                            static_cast<unsigned>(xw == g.lx - 1 ? 0 : xw + 1)};
+    const unsigned ys[3] = {static_cast<unsigned>(yw == 0 ? g.ly - 1 : yw - 1) * g.lx,
+                            static_cast<unsigned>(yw) * g.lx,
+                            static_cast<unsigned>(yw == g.ly - 1 ? 0 : yw + 1) * g.lx};
 
     float a[Q];
     float a_om = 0.f, a_s = 0.f;
@@ -516,44 +505,51 @@ __device__ __forceinline__ void sweep2_run(const Geom& g, int x0, int y0, int z0
     auto prefetch = [&](int zz) {        // issue sweep k's pulls for plane zz
         if (!owner) return;
         const int zw = zz < 0 ? zz + g.lz : (zz >= g.lz ? zz - g.lz : zz);
-        pull_regs32(a, hin, n, g, xw, yw, zw);
-        const int c = (zw * g.ly + yw) * g.lx + xw;
+        const unsigned zs[3] = {(zw == 0 ? g.lz - 1 : zw - 1) * plane, zw * plane, (zw == g.lz - 1 ? 0 : zw + 1) * plane};
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            a[q] = __ldg(hin + (q * n + zs[1 - cz(q)] + (ys[1 - cy(q)] + xs[1 - cx(q)])));
+        });
+        const unsigned c = zs[1] + ys[1] + xs[1];
         a_om = __ldg(omega + c);
         if constexpr (kRefine) {
-            static_for<0, Q>([&](auto qc) { ar[decltype(qc)::value] = __ldg(s + decltype(qc)::value * n + c); });
+            static_for<0, Q>([&](auto qc) { ar[decltype(qc)::value] = __ldg(s + (decltype(qc)::value * n + c)); });
         } else {
             a_s = __ldg(s + c);
         }
     };
-    auto finish = [&](int zz) {          // complete sweep k on plane zz into the ring
+    auto finish = [&](int i) {           // complete sweep k on plane z0 - 1 + i into the ring
         if (!owner) return;
         bounce_regs(a, g, xw);
+        float* cf = coef + (i & 1) * 2 * RC + t;
+        cf[0] = a_om;
         if constexpr (kRefine) {
             const float pe = refine_sum(a);
             static_for<0, Q>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
-                ring[ring_plane<q>(zz) * RC + t] = refine_cell<q>(a[q], pe, a_om, ar[q]);
+                ring[ring_plane<q>(i) * RC + t] = refine_cell<q>(a[q], pe, a_om, ar[q]);
             });
         } else {
-            const P32 p32 = sum_q32(a);
+            cf[RC] = a_s;
+            const P32Hi p32 = sum_q32(a);
             static_for<0, Q>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
-                ring[ring_plane<q>(zz) * RC + t] = collide_h<q>(a[q], p32, a_om, a_s);
+                ring[ring_plane<q>(i) * RC + t] = collide_h<q>(a[q], p32, a_om, a_s);
             });
         }
     };
 
     prefetch(z0 - 1);
-    finish(z0 - 1);
+    finish(0);
     prefetch(z0);
-    finish(z0);
+    finish(1);
     prefetch(z0 + 1);
-    const int tx = t % TX, ty = t / TX;
-    const int x = x0 + tx, y = y0 + ty;
-    const int rc = (ty + 1) * RX + (tx + 1);
+    const int x = x0 + t % TX, y = y0 + t / TX;
+    const int rc = (t / TX + 1) * RX + (t % TX + 1);
     const bool inner = t < TX * TY && x < g.lx && y < g.ly;
     for (int z = z0; z < z1; ++z) {
-        finish(z + 1);
+        const int i = z - z0 + 1;
+        finish(i + 1);
         if (z + 1 < z1) prefetch(z + 2);
         __syncthreads();
         if (inner) {
@@ -561,21 +557,28 @@ __device__ __forceinline__ void sweep2_run(const Geom& g, int x0, int y0, int z0
             float hv[Q];
             static_for<0, Q>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
-                hv[q] = ring[ring_plane<q>(z - cz(q)) * RC + rc - cy(q) * RX - cx(q)];
+                hv[q] = ring[ring_plane<q>(i - cz(q)) * RC + rc - cy(q) * RX - cx(q)];
             });
+            const float* cf = coef + (i & 1) * 2 * RC + rc;
             bounce_regs(hv, g, x);
-            const int c = (z * g.ly + y) * g.lx + x;
+            const unsigned c = z * plane + static_cast<unsigned>(y * g.lx + x);
             if constexpr (kRefine) {
                 const float pe = refine_sum(hv);
-                const float om = __ldg(omega + c);
+                const float om = cf[0];
                 static_for<0, Q>([&](auto qc) {
                     constexpr int q = decltype(qc)::value;
-                    hout[q * n + c] = refine_cell<q>(hv[q], pe, om, __ldg(s + q * n + c));
+                    hout[q * n + c] = refine_cell<q>(hv[q], pe, om, __ldg(s + (q * n + c)));
                 });
             } else {
-                collide_h_store32(hv, sum_q32(hv), __ldg(omega + c), __ldg(s + c), hout, n, c);
+                const P32Hi p32 = sum_q32(hv);
+                const float om = cf[0], sv = cf[RC];
+                static_for<0, Q>([&](auto qc) {
+                    constexpr int q = decltype(qc)::value;
+                    hout[q * n + c] = collide_h<q>(hv[q], p32, om, sv);
+                });
             }
         }
+        __syncthreads();
     }
 }
 

@@ -7,10 +7,9 @@
 // warp per row) for the whole march.  Per plane it completes sweep k at its
 // cell of plane z+1 into a shared-memory plane ring, issues the pulls of plane
 // z+2 (in flight while the CTA works from the ring), and after a barrier
-// computes sweep k+1 of plane z at its own cell from the ring; a second barrier
-// frees the slots that the next plane overwrites, so population q needs
-// cz(q) + 2 slots (30 population planes).  A cell's coefficients are kept beside
-// the ring for sweep k+1.  Coordinates wrap, so the stream and the slip overwrite
+// computes sweep k+1 of plane z at its own cell from the ring (lbm_device.cuh); a
+// second barrier frees the slots that the next plane overwrites.  A cell's
+// coefficients are kept beside the ring for sweep k+1.  Coordinates wrap, so the stream and the slip overwrite
 // are those of two single launches for any box.  Cells outside the box
 // (partial tiles) store nothing.  15 n < 2^31 is required (the launchers check).
 //
@@ -33,7 +32,7 @@ namespace lbm {
 constexpr int F2_RX = 32, F2_RY = 8;                     // region: tile and halo
 constexpr int F2_TX = F2_RX - 2, F2_TY = F2_RY - 2;      // tile
 constexpr int F2_RC = F2_RX * F2_RY;
-constexpr int F2_PLANES = 30;
+constexpr int F2_PLANES = ring_planes();
 constexpr int F2_CTAS = 2;                               // per SM
 // Shared memory with `coefs` coefficients per cell (73,728 B with 3).
 constexpr int f2_smem(int coefs) { return (F2_PLANES + 2 * coefs) * F2_RC * static_cast<int>(sizeof(double)); }
@@ -44,15 +43,6 @@ inline dim3 f2_grid(const Geom& g, int zlen)
 }
 
 namespace {
-
-// Ring plane of population q of plane i (counted from the run's first halo plane).
-template <int q>
-__device__ __forceinline__ int f2_plane(int i)
-{
-    constexpr int slots = cz(q) + 2;
-    constexpr int base = cz(q) < 0 ? 0 : (cz(q) == 0 ? 5 : 15);
-    return base + (i % slots) * 5 + ring_rank(q);
-}
 
 // Ops: fields(c) loads a cell's fields (requested with the pulls), cell(fields)
 // makes its kCoefs coefficients, collide<q>(h, p, coefs) the new population; p
@@ -104,7 +94,7 @@ __device__ __forceinline__ void sweep2_march(const Geom& g, int zlen, const doub
         for (int j = 0; j < K; ++j) cf[j * F2_RC] = k[j];
         static_for<0, Q>([&](auto qc) {
             constexpr int q = decltype(qc)::value;
-            ring[f2_plane<q>(i) * F2_RC + t] = Ops::template collide<q>(a[q], pv, k);
+            ring[ring_plane<q>(i) * F2_RC + t] = Ops::template collide<q>(a[q], pv, k);
         });
     };
 
@@ -123,7 +113,7 @@ __device__ __forceinline__ void sweep2_march(const Geom& g, int zlen, const doub
             double hv[Q];
             static_for<0, Q>([&](auto qc) {
                 constexpr int q = decltype(qc)::value;
-                hv[q] = ring[f2_plane<q>(i - cz(q)) * F2_RC + t - cy(q) * F2_RX - cx(q)];
+                hv[q] = ring[ring_plane<q>(i - cz(q)) * F2_RC + t - cy(q) * F2_RX - cx(q)];
             });
             const double* cf = coef + (i & 1) * K * F2_RC + t;
             double k[K];
