@@ -20,24 +20,46 @@ __device__ __forceinline__ double relative(double num, double den)
 
 // Sums T columns of a partials array (column t at part[t * stride], `count`
 // entries) in a fixed order: thread i adds entries i, i + blockDim, ...
-// sequentially, then a fixed tree (blockDim a power of two <= 1024).
+// sequentially, then a fixed tree, thread i adding the sum of thread i + half
+// for half = blockDim / 2 down to 1 (blockDim a power of two, 32 to 1024; the
+// last five levels within the first warp).  All columns go through the tree
+// together: its barriers are most of a finalisation's time.  sm: scratch of
+// the block (kFinalizeTerms columns).
+constexpr int kFinalizeTerms = 5;
+
 template <int T>
 __device__ void reduce_partials(const double* __restrict__ part, long long stride, long long count,
-                                double (&out)[T])
+                                double (&out)[T], double (&sm)[kFinalizeTerms][1024])
 {
-    __shared__ double sm[1024];
+    static_assert(T <= kFinalizeTerms, "columns of the scratch");
+    double acc[T];
+#pragma unroll
     for (int t = 0; t < T; ++t) {
-        double acc = 0.0;
-        for (long long i = threadIdx.x; i < count; i += blockDim.x) acc += part[t * stride + i];
-        sm[threadIdx.x] = acc;
-        __syncthreads();
-        for (int half = blockDim.x / 2; half > 0; half >>= 1) {
-            if (threadIdx.x < half) sm[threadIdx.x] += sm[threadIdx.x + half];
-            __syncthreads();
+        acc[t] = 0.0;
+        for (long long i = threadIdx.x; i < count; i += blockDim.x) acc[t] += part[t * stride + i];
+        sm[t][threadIdx.x] = acc[t];
+    }
+    __syncthreads();
+    for (int half = blockDim.x / 2; half >= 32; half >>= 1) {
+        if (threadIdx.x < half) {
+#pragma unroll
+            for (int t = 0; t < T; ++t) sm[t][threadIdx.x] += sm[t][threadIdx.x + half];
         }
-        out[t] = sm[0];
         __syncthreads();
     }
+    if (threadIdx.x < 32) {
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            double s = sm[t][threadIdx.x];
+#pragma unroll
+            for (int half = 16; half > 0; half >>= 1) s += __shfl_down_sync(0xffffffffu, s, half);
+            if (threadIdx.x == 0) sm[t][0] = s;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < T; ++t) out[t] = sm[t][0];
+    __syncthreads();
 }
 
 __device__ __forceinline__ void set_error(DevState* ds, int site)
@@ -55,10 +77,11 @@ __device__ void finalize_body(int kind, DevState* __restrict__ ds, const double*
                               long long stride, long long count, const double* __restrict__ part2,
                               long long stride2, long long count2)
 {
+    __shared__ double sm[kFinalizeTerms][1024];
     const double n = ds->n_cells;
     if (kind == FIN_SOURCE) {
         double r[3];
-        reduce_partials<3>(part, stride, count, r);
+        reduce_partials<3>(part, stride, count, r, sm);
         if (threadIdx.x == 0) {
             ds->div_sum = r[0];
             ds->div_abs_sum = r[1];
@@ -67,7 +90,7 @@ __device__ void finalize_body(int kind, DevState* __restrict__ ds, const double*
         }
     } else if (kind == FIN_PREP) {
         double r[3];
-        reduce_partials<3>(part, stride, count, r);
+        reduce_partials<3>(part, stride, count, r, sm);
         if (threadIdx.x == 0) {
             ds->proj_sum = r[0];
             if (r[1] != 0.0 || !isfinite(r[0])) set_error(ds, SITE_PROJECTED);
@@ -79,7 +102,7 @@ __device__ void finalize_body(int kind, DevState* __restrict__ ds, const double*
         }
     } else if (kind == FIN_SIGMA) {
         double r[1];
-        reduce_partials<1>(part, stride, count, r);
+        reduce_partials<1>(part, stride, count, r, sm);
         if (threadIdx.x == 0) {
             const double shift = r[0] / n - ds->target;
             if (!isfinite(shift)) set_error(ds, SITE_GAUGE_SHIFT);
@@ -88,9 +111,9 @@ __device__ void finalize_body(int kind, DevState* __restrict__ ds, const double*
         }
     } else if (kind == FIN_CHECK) {
         double rb[5];
-        reduce_partials<5>(part, stride, count, rb);
+        reduce_partials<5>(part, stride, count, rb, sm);
         double rc[3] = {0.0, 0.0, 0.0};
-        if (ds->dual) reduce_partials<3>(part2, stride2, count2, rc);
+        if (ds->dual) reduce_partials<3>(part2, stride2, count2, rc, sm);
         if (threadIdx.x == 0) {
             bool fp_ok = true;
             if (ds->dual) {
@@ -121,15 +144,15 @@ __device__ void finalize_body(int kind, DevState* __restrict__ ds, const double*
         }
     } else if (kind == FIN_MASS) {
         double r[1];
-        reduce_partials<1>(part, stride, count, r);
+        reduce_partials<1>(part, stride, count, r, sm);
         if (threadIdx.x == 0) ds->mass = r[0];
     } else if (kind == FIN_BLOCK) {
         double r[1];
-        reduce_partials<1>(part, stride, count, r);
+        reduce_partials<1>(part, stride, count, r, sm);
         if (threadIdx.x == 0) ds->block_frac = ds->l1_delta > 0.0 ? r[0] / ds->l1_delta : 0.0;
     } else if (kind == FIN_RHS) {
         double r[3];
-        reduce_partials<3>(part, stride, count, r);
+        reduce_partials<3>(part, stride, count, r, sm);
         if (threadIdx.x == 0) {
             ds->rhs_mean = r[0] / r[2];
             ds->rhs_chk = r[1] / r[2];

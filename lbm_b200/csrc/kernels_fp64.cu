@@ -48,11 +48,12 @@ namespace {
 // Tile of a check kernel: planes [blockIdx.z * zrun, +zrun) of one 2-D tile,
 // so the CTA's block reduction and its loads of the device-side scalars are
 // amortised over zrun planes.
+template <int kPlanes = 1>
 __device__ __forceinline__ bool tile_zrun(const Geom& g, int zrun, int& x, int& y, int& z0, int& z1)
 {
     x = blockIdx.x * blockDim.x + threadIdx.x;
     y = blockIdx.y * blockDim.y + threadIdx.y;
-    z0 = blockIdx.z * zrun;
+    z0 = blockIdx.z / kPlanes * zrun;
     z1 = min(z0 + zrun, g.lz);
     return x < g.lx && y < g.ly;
 }
@@ -511,14 +512,15 @@ sweep2_kernel(Geom g, int zlen, const double* __restrict__ hin, double* __restri
     sweep2_march(g, zlen, hin, hout, SweepOps{rho, s}, ring);
 }
 
-__global__ void __launch_bounds__(256)
+template <int kPlanes>
+__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
 sweep_check_a_kernel(Geom g, int zrun, const double* __restrict__ hin, double* __restrict__ hout,
                      double* __restrict__ p_chk, double* __restrict__ part, long long nblocks)
 {
     int x, y, z0, z1;
-    const bool active = tile_zrun(g, zrun, x, y, z0, z1);
+    const bool active = tile_zrun<kPlanes>(g, zrun, x, y, z0, z1);
     double red[1] = {0.0};
-    for (int z = z0; active && z < z1; ++z) {
+    const bool reduce = zrun_terms<kPlanes, 1>(z0, z1, active, red, [&](int z, double (&r)[1]) {
         const long long c = cell_of(g, x, y, z);
         double hv[Q];
         pull_regs(hv, hin, g, x, y, z);
@@ -529,13 +531,13 @@ sweep_check_a_kernel(Geom g, int zrun, const double* __restrict__ hin, double* _
             hout[(long long)q * g.n + c] = hv[q];
         });
         p_chk[c] = pv;
-        red[0] += pv;
-    }
-    block_sum_store<1>(red, part, nblocks, block_linear());
+        r[0] += pv;
+    });
+    if (reduce) block_sum_store<1>(red, part, nblocks, run_linear<kPlanes>());
 }
 
-template <bool kDual>
-__global__ void __launch_bounds__(256)
+template <bool kDual, int kPlanes>
+__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
 sweep_check_b_kernel(Geom g, int zrun, const double* __restrict__ hin, double* __restrict__ hout,
                      double* __restrict__ hc,
                      const double* __restrict__ p_chk, double* __restrict__ p_prev,
@@ -544,11 +546,11 @@ sweep_check_b_kernel(Geom g, int zrun, const double* __restrict__ hin, double* _
                      double* __restrict__ part, long long nblocks)
 {
     int x, y, z0, z1;
-    const bool active = tile_zrun(g, zrun, x, y, z0, z1);
+    const bool active = tile_zrun<kPlanes>(g, zrun, x, y, z0, z1);
     double red[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     const double shift = ds->sigma;
     const double tgt = ds->target;
-    for (int z = z0; active && z < z1; ++z) {
+    const bool reduce = zrun_terms<kPlanes, kDual ? 5 : 2>(z0, z1, active, red, [&](int z, double (&r)[5]) {
         const long long c = cell_of(g, x, y, z);
         double hv[Q];
         // Gauge (CPU/Inamuro.cpp:699-705): p -= shift, h_q -= E_q shift.
@@ -563,19 +565,19 @@ sweep_check_b_kernel(Geom g, int zrun, const double* __restrict__ hin, double* _
                 hc[(long long)q * g.n + c] = hv[q];
             });
             const double hsum = sum_q(hv);
-            red[2] += fabs(pv - hsum);
-            red[3] += fabs(pv - tgt);
-            red[4] += fabs(hsum - tgt);
+            r[2] += fabs(pv - hsum);
+            r[3] += fabs(pv - tgt);
+            r[4] += fabs(hsum - tgt);
         }
         // Relative change (CPU/Inamuro.cpp:726-753).
-        red[0] += fabs(pv - p_prev[c]);
-        red[1] += fabs(pv);
+        r[0] += fabs(pv - p_prev[c]);
+        r[1] += fabs(pv);
         p_prev[c] = pv;
         p[c] = pv;
         const double tauh = 1.0 / __ldg(rho + c) + 0.5;
         collide_h_store(hv, pv, tauh, __ldg(s + c), hout, g.n, c);
-    }
-    block_sum_store<5>(red, part, nblocks, block_linear());
+    });
+    if (reduce) block_sum_store<5>(red, part, nblocks, run_linear<kPlanes>());
 }
 
 __global__ void __launch_bounds__(256)
@@ -1129,19 +1131,22 @@ void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double*
 void sweep_check_a(cudaStream_t st, const Launch& L, const Geom& g, const double* hin,
                    double* hout, double* p_chk, double* part)
 {
-    sweep_check_a_kernel<<<L.cgrid, L.block, 0, st>>>(g, L.zrun, hin, hout, p_chk, part, L.cnblocks);
+    const bool planes = L.cnblocks < kCheckPlaneRuns;
+    auto kern = planes ? sweep_check_a_kernel<kCheckZrun> : sweep_check_a_kernel<1>;
+    kern<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, hin, hout, p_chk, part, L.cnblocks);
 }
 
 void sweep_check_b(cudaStream_t st, const Launch& L, const Geom& g, bool dual, const double* hin, double* hout,
                    double* hc, const double* p_chk, double* p_prev, double* p, const double* rho,
                    const double* s, const DevState* ds, double* part)
 {
-    if (dual)
-        sweep_check_b_kernel<true><<<L.cgrid, L.block, 0, st>>>(g, L.zrun, hin, hout, hc, p_chk, p_prev, p, rho,
-                                                                s, ds, part, L.cnblocks);
-    else
-        sweep_check_b_kernel<false><<<L.cgrid, L.block, 0, st>>>(g, L.zrun, hin, hout, hc, p_chk, p_prev, p, rho,
-                                                                 s, ds, part, L.cnblocks);
+    // (five terms of eight planes are more than a CTA's static shared memory)
+    const bool planes = !dual && L.cnblocks < kCheckPlaneRuns;
+    auto kern = dual     ? sweep_check_b_kernel<true, 1>
+                : planes ? sweep_check_b_kernel<false, kCheckZrun>
+                         : sweep_check_b_kernel<false, 1>;
+    kern<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, hin, hout, hc, p_chk, p_prev, p, rho, s, ds, part,
+                                                   L.cnblocks);
 }
 
 void sweep_check_c(cudaStream_t st, const Launch& L, const Geom& g, const double* hin,

@@ -29,11 +29,12 @@ namespace {
 // Tile of a check kernel: planes [blockIdx.z * zrun, +zrun) of one 2-D tile,
 // so the CTA's block reduction and its loads of the device-side scalars are
 // amortised over zrun planes.
+template <int kPlanes = 1>
 __device__ __forceinline__ bool tile_zrun(const Geom& g, int zrun, int& x, int& y, int& z0, int& z1)
 {
     x = blockIdx.x * blockDim.x + threadIdx.x;
     y = blockIdx.y * blockDim.y + threadIdx.y;
-    z0 = blockIdx.z * zrun;
+    z0 = blockIdx.z / kPlanes * zrun;
     z1 = min(z0 + zrun, g.lz);
     return x < g.lx && y < g.ly;
 }
@@ -221,19 +222,21 @@ sweep2_refine_kernel(Geom g, int zlen, const float* __restrict__ ein, float* __r
                                      omega, r, ring);
 }
 
-__global__ void __launch_bounds__(256)
+template <int kPlanes>
+__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
 sweep_check_a_kernel(Geom g, int zrun, const float* __restrict__ hin, float* __restrict__ hout,
                      double* __restrict__ p_chk, double* __restrict__ part, long long nblocks)
 {
     int x, y, z0, z1;
-    const bool active = tile_zrun(g, zrun, x, y, z0, z1);
+    const bool active = tile_zrun<kPlanes>(g, zrun, x, y, z0, z1);
     double red[1] = {0.0};
-    for (int z = z0; active && z < z1; ++z) mixc_check_a(g, hin, hout, p_chk, x, y, z, red);
-    block_sum_store<1>(red, part, nblocks, block_linear());
+    const bool reduce = zrun_terms<kPlanes, 1>(z0, z1, active, red,
+                          [&](int z, double (&r)[1]) { mixc_check_a(g, hin, hout, p_chk, x, y, z, r); });
+    if (reduce) block_sum_store<1>(red, part, nblocks, run_linear<kPlanes>());
 }
 
-template <bool kDual>
-__global__ void __launch_bounds__(256)
+template <bool kDual, int kPlanes>
+__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
 sweep_check_b_kernel(Geom g, int zrun, const float* __restrict__ hin, float* __restrict__ hout,
                      float* __restrict__ hc,
                      const double* __restrict__ p_chk, double* __restrict__ p_prev,
@@ -242,13 +245,14 @@ sweep_check_b_kernel(Geom g, int zrun, const float* __restrict__ hin, float* __r
                      double* __restrict__ part, long long nblocks)
 {
     int x, y, z0, z1;
-    const bool active = tile_zrun(g, zrun, x, y, z0, z1);
+    const bool active = tile_zrun<kPlanes>(g, zrun, x, y, z0, z1);
     double red[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     const double shift = ds->sigma;
     const double tgt = ds->target;
-    for (int z = z0; active && z < z1; ++z)
-        mixc_check_b<kDual>(g, hin, hout, hc, p_chk, p_prev, p, omega, s, shift, tgt, x, y, z, red);
-    block_sum_store<5>(red, part, nblocks, block_linear());
+    const bool reduce = zrun_terms<kPlanes, kDual ? 5 : 2>(z0, z1, active, red, [&](int z, double (&r)[5]) {
+        mixc_check_b<kDual>(g, hin, hout, hc, p_chk, p_prev, p, omega, s, shift, tgt, x, y, z, r);
+    });
+    if (reduce) block_sum_store<5>(red, part, nblocks, run_linear<kPlanes>());
 }
 
 __global__ void __launch_bounds__(256)
@@ -363,15 +367,16 @@ refine_sweep_kernel(Geom g, const float* __restrict__ ein, float* __restrict__ e
 
 // Check A in FP64: pull H + e, slip, p = sum (FP64); the uncollided values
 // go to hpre, red[0] += p.
-__global__ void __launch_bounds__(256)
+template <int kPlanes>
+__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
 refine_check_a_kernel(Geom g, int zrun, const double* __restrict__ hd, const float* __restrict__ e,
                       double* __restrict__ hpre, double* __restrict__ p_chk, double* __restrict__ part,
                       long long nblocks)
 {
     int x, y, z0, z1;
-    const bool active = tile_zrun(g, zrun, x, y, z0, z1);
+    const bool active = tile_zrun<kPlanes>(g, zrun, x, y, z0, z1);
     double red[1] = {0.0};
-    for (int z = z0; active && z < z1; ++z) {
+    const bool reduce = zrun_terms<kPlanes, 1>(z0, z1, active, red, [&](int z, double (&r)[1]) {
         const long long c = cell_of(g, x, y, z);
         const Wrap w(g, x, y, z);
         double hv[Q];
@@ -388,28 +393,29 @@ refine_check_a_kernel(Geom g, int zrun, const double* __restrict__ hd, const flo
             hpre[(long long)q * g.n + c] = hv[q];
         });
         p_chk[c] = pv;
-        red[0] += pv;
-    }
-    block_sum_store<1>(red, part, nblocks, block_linear());
+        r[0] += pv;
+    });
+    if (reduce) block_sum_store<1>(red, part, nblocks, run_linear<kPlanes>());
 }
 
 // Check B in FP64: gauge (p -= shift, h -= E shift), relative-change terms,
 // p and p_prev, then the collision of the next sweep, in place.
-__global__ void __launch_bounds__(256)
+template <int kPlanes>
+__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
 refine_check_b_kernel(Geom g, int zrun, double* __restrict__ hd, const double* __restrict__ p_chk,
                       double* __restrict__ p_prev, double* __restrict__ p, const float* __restrict__ omega,
                       const float* __restrict__ s, const DevState* __restrict__ ds, double* __restrict__ part,
                       long long nblocks)
 {
     int x, y, z0, z1;
-    const bool active = tile_zrun(g, zrun, x, y, z0, z1);
+    const bool active = tile_zrun<kPlanes>(g, zrun, x, y, z0, z1);
     double red[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     const double shift = ds->sigma;
-    for (int z = z0; active && z < z1; ++z) {
+    const bool reduce = zrun_terms<kPlanes, 2>(z0, z1, active, red, [&](int z, double (&r)[5]) {
         const long long c = cell_of(g, x, y, z);
         const double pv = p_chk[c] - shift;
-        red[0] += fabs(pv - p_prev[c]);
-        red[1] += fabs(pv);
+        r[0] += fabs(pv - p_prev[c]);
+        r[1] += fabs(pv);
         p_prev[c] = pv;
         p[c] = pv;
         const double om = __ldg(omega + c), sv = __ldg(s + c);
@@ -419,8 +425,8 @@ refine_check_b_kernel(Geom g, int zrun, double* __restrict__ hd, const double* _
             const double hv = hd[i] - wE(q) * shift;
             hd[i] = hv - om * (hv - wE(q) * pv) - wE(q) / 3.0 * sv;
         });
-    }
-    block_sum_store<5>(red, part, nblocks, block_linear());
+    });
+    if (reduce) block_sum_store<5>(red, part, nblocks, run_linear<kPlanes>());
 }
 
 __global__ void __launch_bounds__(256)
@@ -680,18 +686,18 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
             sweep_kernel64<<<L.grid, L.block, 0, st>>>(g, mb.h[cur], mb.h[1 - cur], omega, mb.s);
         cur = 1 - cur;
     }
-    sweep_check_a_kernel<<<L.cgrid, L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.p_chk, mb.part_a,
-                                                      L.cnblocks);
+    bool planes = L.cnblocks < kCheckPlaneRuns;
+    auto check_a = planes ? sweep_check_a_kernel<kCheckZrun> : sweep_check_a_kernel<1>;
+    check_a<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.p_chk, mb.part_a, L.cnblocks);
     cur = 1 - cur;
     finalize(st, FIN_SIGMA, ds, mb.part_a, L.cnblocks, nullptr, 0, nullptr, 0);
-    if (dual)
-        sweep_check_b_kernel<true><<<L.cgrid, L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.hc,
-                                                                mb.p_chk, mb.p_prev, mb.p, omega, mb.s, ds,
-                                                                mb.part_b, L.cnblocks);
-    else
-        sweep_check_b_kernel<false><<<L.cgrid, L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.hc,
-                                                                 mb.p_chk, mb.p_prev, mb.p, omega, mb.s, ds,
-                                                                 mb.part_b, L.cnblocks);
+    // (five terms of eight planes are more than a CTA's static shared memory)
+    planes = planes && !dual;
+    auto check_b = dual     ? sweep_check_b_kernel<true, 1>
+                   : planes ? sweep_check_b_kernel<false, kCheckZrun>
+                            : sweep_check_b_kernel<false, 1>;
+    check_b<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.hc, mb.p_chk, mb.p_prev,
+                                                      mb.p, omega, mb.s, ds, mb.part_b, L.cnblocks);
     cur = 1 - cur;
     if (dual) {
         sweep_check_c_kernel<<<L.cgrid, L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.hc, omega, mb.s,
@@ -761,10 +767,13 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
         cur = 1 - cur;
     }
     // the check sweep in FP64 on H + e
-    refine_check_a_kernel<<<L.cgrid, L.block, 0, st>>>(g, L.zrun, H, e, Hn, mb.p_chk, mb.part_a, L.cnblocks);
+    const bool planes = L.cnblocks < kRefinePlaneRuns;
+    auto check_a = planes ? refine_check_a_kernel<kCheckZrun> : refine_check_a_kernel<1>;
+    check_a<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, H, e, Hn, mb.p_chk, mb.part_a, L.cnblocks);
     finalize(st, FIN_SIGMA, ds, mb.part_a, L.cnblocks, nullptr, 0, nullptr, 0);
-    refine_check_b_kernel<<<L.cgrid, L.block, 0, st>>>(g, L.zrun, Hn, mb.p_chk, mb.p_prev, mb.p, omega, mb.s, ds,
-                                                       mb.part_b, L.cnblocks);
+    auto check_b = planes ? refine_check_b_kernel<kCheckZrun> : refine_check_b_kernel<1>;
+    check_b<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, Hn, mb.p_chk, mb.p_prev, mb.p, omega, mb.s, ds,
+                                                      mb.part_b, L.cnblocks);
     finalize(st, FIN_CHECK, ds, mb.part_b, L.cnblocks, nullptr, 0, nullptr, 0);
     return 1 - start_parity;
 }

@@ -8,6 +8,8 @@
 // at compile time, with no constant-memory traffic.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include <cstdint>
 #include <type_traits>
 #include <utility>
@@ -340,9 +342,49 @@ __device__ __forceinline__ void block_sum_store(double (&v)[T], double* __restri
     }
 }
 
+// Terms of a check kernel's cells over a run of up to 8 planes from z0 of its
+// tile: cell(z, r) adds plane z's to r; true where the caller is to reduce red.
+// kPlanes 1: a thread takes its column's planes [z0, z1) in turn.  kPlanes 8: the
+// run is a cluster of eight CTAs, one plane each (grid z 8 times as long); each
+// hands its terms to the first, which adds them in the same order, so red is
+// bitwise the same (a cell adds at most one value to a term).
+template <int kPlanes, int T, int R, class F>
+__device__ __forceinline__ bool zrun_terms(int z0, int z1, bool active, double (&red)[R], F&& cell)
+{
+    if constexpr (kPlanes == 1) {
+        for (int z = z0; active && z < z1; ++z) cell(z, red);
+        return true;
+    } else {
+        __shared__ double terms[T][kPlanes][256];
+        const auto cluster = cooperative_groups::this_cluster();
+        const int t = threadIdx.x + blockDim.x * threadIdx.y;
+        const int plane = blockIdx.z % kPlanes;
+        auto token = cluster.barrier_arrive();   // (the first CTA has started when its peers write to it)
+        double r[R] = {};
+        if (active && z0 + plane < z1) cell(z0 + plane, r);
+        cluster.barrier_wait(std::move(token));
+        double* to = cluster.map_shared_rank(&terms[0][0][0], 0);
+#pragma unroll
+        for (int i = 0; i < T; ++i) to[(i * kPlanes + plane) * 256 + t] = r[i];
+        cluster.sync();
+        if (plane != 0) return false;
+        for (int z = z0; active && z < z1; ++z)
+#pragma unroll
+            for (int i = 0; i < T; ++i) red[i] += terms[i][z - z0][t];
+        return true;
+    }
+}
+
 __device__ __forceinline__ long long block_linear()
 {
     return blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+}
+
+// The same for a kernel whose runs are clusters of kPlanes CTAs in z.
+template <int kPlanes>
+__device__ __forceinline__ long long run_linear()
+{
+    return blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * (blockIdx.z / kPlanes));
 }
 
 }  // namespace lbm

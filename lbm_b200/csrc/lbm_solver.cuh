@@ -78,7 +78,22 @@ struct Launch {
     dim3 cgrid;
     long long cnblocks;
     int zrun;
+    // Grid of a check kernel that runs a plane per CTA, clusters of kCheckZrun
+    // making a run (zrun_terms); else cgrid.
+    dim3 check_grid(bool planes) const { return planes ? dim3(cgrid.x, cgrid.y, cgrid.z * kCheckZrun) : cgrid; }
 };
+
+// Runs below which checks A and B go a plane per CTA: with one CTA per run a
+// check of a small box is eight planes one after another on a few SMs (32^3: 16
+// CTAs).  Per sweep of a check interval of 100, us, a run per CTA and a plane per
+// CTA: FP64 2.81 and 2.69 at 32^3 (16 runs), 4.26 and 4.20 at 48^3 (72), 7.84
+// both at 64^3 (128), 14.39 and 14.43 at 72^3 (243); FP32 2.08 and 1.95, 2.95 and
+// 2.79, 4.88 and 4.82, 7.10 both, 12.91 and 13.10 at 88^3 (363).
+constexpr long long kCheckPlaneRuns = 148;
+// The refinement form's, in FP64 on H + e: 2.49 and 2.19 at 32^3, 6.18 and 5.90
+// at 64^3, 14.45 and 14.14 at 80^3 (300), 37.1 and 36.9 at 104^3 (676), 59.3 and
+// 59.4 at 128^3 (1024).
+constexpr long long kRefinePlaneRuns = 740;
 
 inline Launch make_launch(int lx, int ly, int lz, int bx, int by)
 {
