@@ -15,7 +15,8 @@
 // parity of its current h buffer, sweep cap).  A segment (check_interval
 // sweeps, check kernels A and B, the per-instance finalisations) is one
 // captured CUDA graph for the whole batch; items of instances that have left
-// the loop are skipped, and each instance's h parity advances only while it is
+// the loop are skipped (the two-sweep passes' list is rebuilt without them
+// before each segment), and each instance's h parity advances only while it is
 // active.  The segments repeat on the device (a conditional WHILE graph node
 // and b_loop_decide) until no instance is active, at most 64 per launch; the
 // host reads the control words once per launch and relaunches while any
@@ -184,25 +185,90 @@ b_sweep(const BItem* __restrict__ items, int n_items, const BInst* __restrict__ 
     }
 }
 
-// Two plain sweeps (flip index j: state in h[(parity + j) & 1], result in the
-// other buffer) for every active instance, 16 x 8 tiles with temporal
-// blocking (sweep2_run).
-constexpr int B2_TX = 16, B2_TY = 8;
-constexpr int B2_THREADS = sweep2_threads(B2_TX, B2_TY);   // 192
-constexpr int B2_SMEM = sweep2_smem(B2_TX, B2_TY);         // 24,480 B
-constexpr int B2_CTAS_PER_SM = 4;
+// Two-sweep passes: 32 x 8 tiles, two CTAs an SM.  us per sweep of ten boxes of
+// 48 to 96 cells a side (3.77 million cells), all, five and two of them in their
+// loops: 60.9, 31.3, 16.6, against 66.3, 33.9, 17.7 with 16 x 16 tiles, 67.7, 34.2,
+// 16.1 with 16 x 8 (four CTAs), 61.4, 33.0, 16.7 with 32 x 16 (one CTA) and 70 to
+// 76 with 30 x 8, 30 x 14, 16 x 32 and 14 x 14.
+constexpr int B2_TX = 32, B2_TY = 8;
+constexpr int B2_THREADS = sweep2_threads(B2_TX, B2_TY);   // 352
+constexpr int B2_SMEM = sweep2_smem(B2_TX, B2_TY);         // 46,240 B
+constexpr int B2_CTAS_PER_SM = 2;
+constexpr int kPlanRuns = 64;      // longest run (sweep2_zrun's limit)
+constexpr int kPlanShortest = 4;   // shortest, unless sweep2_zrun is below it
 
+__device__ __forceinline__ int b2_tiles(const Geom& g)
+{
+    return ((g.lx + B2_TX - 1) / B2_TX) * ((g.ly + B2_TY - 1) / B2_TY);
+}
+
+// Work list of the two-sweep passes of a segment, rebuilt before it: the items
+// of the instances still in their loops, without gaps, so that the CTAs of the
+// passes have the same share whichever instances have left.  An instance's
+// column of tiles is cut into runs of equal length, at most zmax planes: the
+// length for which the passes' waves (items over `slots` resident CTAs) times
+// the planes a CTA works through (its run and two halo planes) is least.
+// One CTA per instance; each finds the length and its own offset (a few us per
+// segment).  With a fixed list whose items of instances that have left are
+// skipped: 38.5 us per sweep with five of the ten boxes left and 23.4 with two.
+__global__ void __launch_bounds__(256)
+b_plan2(const BInst* __restrict__ inst, const BCtl* __restrict__ ctl, int n, int zmax, int slots,
+        BItem* __restrict__ items, int* __restrict__ n_items)
+{
+    __shared__ int total[kPlanRuns + 1];
+    __shared__ int best, first;
+    const int me = blockIdx.x;
+    for (int z = threadIdx.x; z <= kPlanRuns; z += blockDim.x) total[z] = 0;
+    if (threadIdx.x == 0) first = 0;
+    __syncthreads();
+    // thread: one length, every fourth instance
+    const int z = threadIdx.x % kPlanRuns + 1;
+    int mine = 0;
+    for (int i = threadIdx.x / kPlanRuns; i < n; i += 256 / kPlanRuns)
+        if (ctl[i].active) mine += b2_tiles(inst[i].g) * ((inst[i].g.lz + z - 1) / z);
+    atomicAdd(&total[z], mine);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        long long least = 0;
+        best = zmax;
+        for (int k = zmax; k >= 1 && (k >= kPlanShortest || k == zmax); --k) {
+            const long long cost = static_cast<long long>((total[k] + slots - 1) / slots) * (k + 2);
+            if (k == zmax || cost < least) {
+                best = k;
+                least = cost;
+            }
+        }
+    }
+    __syncthreads();
+    int before = 0;
+    for (int i = threadIdx.x; i < me; i += blockDim.x)
+        if (ctl[i].active) before += b2_tiles(inst[i].g) * ((inst[i].g.lz + best - 1) / best);
+    atomicAdd(&first, before);
+    __syncthreads();
+    if (me == 0 && threadIdx.x == 0) *n_items = total[best];
+    if (!ctl[me].active) return;
+    const Geom g = inst[me].g;
+    const int nx = (g.lx + B2_TX - 1) / B2_TX, per = b2_tiles(g);
+    // (len <= best, so that (nz - 1) len < lz: no run is empty)
+    const int nz = (g.lz + best - 1) / best, len = (g.lz + nz - 1) / nz;
+    for (int k = threadIdx.x; k < per * nz; k += blockDim.x) {
+        const int r = k % per, z0 = k / per * len;
+        items[first + k] = BItem{me, r % nx * B2_TX, r / nx * B2_TY, z0, min(z0 + len, g.lz)};
+    }
+}
+
+// Two plain sweeps (flip index j: state in h[(parity + j) & 1], result in the
+// other buffer) for every item of the plan, with temporal blocking (sweep2_run).
 __global__ void __launch_bounds__(B2_THREADS, B2_CTAS_PER_SM)
-b_sweep2(const BItem* __restrict__ items, int n_items, const BInst* __restrict__ inst,
+b_sweep2(const BItem* __restrict__ items, const int* __restrict__ n_items, const BInst* __restrict__ inst,
          const BCtl* __restrict__ ctl, int j, BPool B)
 {
     extern __shared__ float ring[];
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+    const int count = *n_items;
+    for (int it = blockIdx.x; it < count; it += gridDim.x) {
         const BItem w = items[it];
-        const BCtl cw = ctl[w.inst];
-        if (!cw.active) continue;
         const BInst I = inst[w.inst];
-        const bool odd = ((cw.parity + j) & 1) != 0;
+        const bool odd = ((ctl[w.inst].parity + j) & 1) != 0;
         const float* hin = (odd ? B.h[1] : B.h[0]) + I.pop;
         float* hout = (odd ? B.h[0] : B.h[1]) + I.pop;
         sweep2_run<B2_TX, B2_TY>(I.g, w.x0, w.y0, w.z0, w.z1, hin, hout, B.omega + I.fld, B.s + I.fld, ring);
@@ -380,7 +446,7 @@ struct lbm_batch {
     long long pop_elems = 0;         // elements of one pooled population buffer
     long long item_capacity = 0;     // partial-sum slots allocated (largest work list of any tuning)
     int n_items = 0;
-    int n_items2 = 0;                // two-sweep work list (16 x 8 tiles, sweep2_zrun)
+    int* n_items2_d = nullptr;       // two-sweep work list of the running segment (b_plan2)
     BInst* inst_d = nullptr;
     BItem* items_d = nullptr;
     BItem* items2_d = nullptr;
@@ -457,23 +523,6 @@ lbm_status build_items(lbm_batch* b)
     b->items_d = nullptr;
     BCUDA(b, cudaMalloc(&b->items_d, items.size() * sizeof(BItem)));
     BCUDA(b, cudaMemcpy(b->items_d, items.data(), items.size() * sizeof(BItem), cudaMemcpyHostToDevice));
-    // the two-sweep list: 16 x 8 tiles, z runs of sweep2_zrun (no partial sums)
-    std::vector<BItem> items2;
-    if (t.sweep2_zrun > 0)
-        for (int i = 0; i < b->n; ++i) {
-            const BInst& I = b->inst_h[i];
-            for (int z0 = 0; z0 < I.g.lz; z0 += t.sweep2_zrun)
-                for (int y0 = 0; y0 < I.g.ly; y0 += B2_TY)
-                    for (int x0 = 0; x0 < I.g.lx; x0 += B2_TX)
-                        items2.push_back(BItem{i, x0, y0, z0, std::min(z0 + t.sweep2_zrun, I.g.lz)});
-        }
-    b->n_items2 = static_cast<int>(items2.size());
-    if (b->items2_d) cudaFree(b->items2_d);
-    b->items2_d = nullptr;
-    if (!items2.empty()) {
-        BCUDA(b, cudaMalloc(&b->items2_d, items2.size() * sizeof(BItem)));
-        BCUDA(b, cudaMemcpy(b->items2_d, items2.data(), items2.size() * sizeof(BItem), cudaMemcpyHostToDevice));
-    }
     BCUDA(b, cudaMemcpy(b->inst_d, b->inst_h.data(), b->n * sizeof(BInst), cudaMemcpyHostToDevice));
     for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
     b->graphs.clear();
@@ -505,7 +554,9 @@ void free_batch(lbm_batch* b)
     if (b->inst_d) cudaFree(b->inst_d);
     if (b->items_d) cudaFree(b->items_d);
     if (b->items2_d) cudaFree(b->items2_d);
+    if (b->n_items2_d) cudaFree(b->n_items2_d);
     b->items2_d = nullptr;
+    b->n_items2_d = nullptr;
     if (b->ds) cudaFree(b->ds);
     if (b->ctl) cudaFree(b->ctl);
     if (b->ds_host) cudaFreeHost(b->ds_host);
@@ -556,8 +607,22 @@ lbm_status load_instance(lbm_batch* b, int i, const double* const src[6])
     return LBM_OK;
 }
 
-// One segment's kernels on st (a capturing stream): n_normal plain sweeps,
-// check A, FIN_SIGMA, check B, FIN_CHECK.
+// The two-sweep passes' work list for the segment to come, and one pass.
+int grid2_of(const lbm_batch* b) { return B2_CTAS_PER_SM * b->sm_count; }
+
+void enqueue_plan2(lbm_batch* b, cudaStream_t st)
+{
+    b_plan2<<<b->n, 256, 0, st>>>(b->inst_d, b->ctl, b->n, b->tune.sweep2_zrun, grid2_of(b), b->items2_d,
+                                  b->n_items2_d);
+}
+
+void enqueue_sweep2(lbm_batch* b, int j, cudaStream_t st)
+{
+    b_sweep2<<<grid2_of(b), B2_THREADS, B2_SMEM, st>>>(b->items2_d, b->n_items2_d, b->inst_d, b->ctl, j, b->pool);
+}
+
+// One segment's kernels on st (a capturing stream): n_normal plain sweeps
+// (in pairs after b_plan2 when two-sweep passes are on), check A, FIN_SIGMA, check B, FIN_CHECK.
 void enqueue_segment(lbm_batch* b, int n_normal, cudaStream_t st)
 {
     const int grid = grid_of(b);
@@ -565,10 +630,9 @@ void enqueue_segment(lbm_batch* b, int n_normal, cudaStream_t st)
     // j counts buffer swaps: a two-sweep launch swaps once, a single sweep once
     int j = 0;
     int singles = n_normal;
-    if (b->n_items2 > 0) {
-        const int grid2 = std::max(1, std::min(b->n_items2, B2_CTAS_PER_SM * b->sm_count));
-        for (int k = 0; k + 1 < n_normal; k += 2)
-            b_sweep2<<<grid2, B2_THREADS, B2_SMEM, st>>>(b->items2_d, b->n_items2, b->inst_d, b->ctl, j++, b->pool);
+    if (b->tune.sweep2_zrun > 0 && n_normal > 1) {
+        enqueue_plan2(b, st);
+        for (int k = 0; k + 1 < n_normal; k += 2) enqueue_sweep2(b, j++, st);
         singles = n_normal & 1;
     }
     for (int k = 0; k < singles; ++k)
@@ -790,13 +854,15 @@ lbm_status batch_step_once(lbm_batch* b, const uint64_t* replay, lbm_step_stats*
     b->acc.poisson_ms += t[3];
     b->acc.correct_ms += t[4];
     b->acc.steps += 1;
-    // per segment: ci - 1 plain sweeps (in pairs when two-sweep passes are on)
+    // per segment: ci - 1 plain sweeps (in pairs after a plan when two-sweep
+    // passes are on)
     // + check A + check B (together one sweep) + two finalisations; per step:
     // 7 prologue launches and the correction
     b->acc.sweep_kernels += segments * static_cast<uint64_t>(ci + 1);
-    const uint64_t plain = b->n_items2 > 0 ? static_cast<uint64_t>((ci - 1) / 2 + (ci - 1) % 2) : ci - 1;
+    const bool fused = b->tune.sweep2_zrun > 0 && ci > 2;
+    const uint64_t plain = fused ? static_cast<uint64_t>(1 + (ci - 1) / 2 + (ci - 1) % 2) : ci - 1;
     b->acc.kernel_launches += 8 + segments * (plain + 4) + decides;
-    if (b->n_items2 > 0) b->acc.fused_sweeps += segments * static_cast<uint64_t>((ci - 1) / 2 * 2);
+    if (fused) b->acc.fused_sweeps += segments * static_cast<uint64_t>((ci - 1) / 2 * 2);
     lbm_status status = LBM_OK;
     for (int i = 0; i < b->n; ++i) {
         const DevState& d = b->ds_host[i];
@@ -895,6 +961,8 @@ lbm_status lbm_batch_create(const lbm_params* params, int n_instances, int devic
     const long long cap = b->item_capacity;
     ok = ok && okd(&b->part_src, 3 * cap) && okd(&b->part_mass, cap) && okd(&b->part_prep, 3 * cap) &&
          okd(&b->part_a, cap) && okd(&b->part_b, 5 * cap);
+    ok = ok && cudaMalloc(&b->items2_d, count_items(b->prm, B2_TX, B2_TY, 1) * sizeof(BItem)) == cudaSuccess &&
+         cudaMalloc(&b->n_items2_d, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMalloc(&b->inst_d, n_instances * sizeof(BInst)) == cudaSuccess &&
          cudaMalloc(&b->ds, n_instances * sizeof(DevState)) == cudaSuccess &&
          cudaMalloc(&b->ctl, n_instances * sizeof(BCtl)) == cudaSuccess &&
@@ -1068,11 +1136,10 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
         b->tune = t;
         lbm_status s = build_items(b);
         if (s != LBM_OK) return s;
-        const int grid2 = std::max(1, std::min(b->n_items2, B2_CTAS_PER_SM * b->sm_count));
-        b_sweep2<<<grid2, B2_THREADS, B2_SMEM, st>>>(b->items2_d, b->n_items2, b->inst_d, b->ctl, 0, b->pool);
+        enqueue_plan2(b, st);
+        enqueue_sweep2(b, 0, st);
         BCUDA(b, cudaEventRecord(b->ev[0], st));
-        for (int r = 0; r < reps / 2; ++r)
-            b_sweep2<<<grid2, B2_THREADS, B2_SMEM, st>>>(b->items2_d, b->n_items2, b->inst_d, b->ctl, r, b->pool);
+        for (int r = 0; r < reps / 2; ++r) enqueue_sweep2(b, r, st);
         BCUDA(b, cudaEventRecord(b->ev[1], st));
         BCUDA(b, cudaGetLastError());
         BCUDA(b, cudaEventSynchronize(b->ev[1]));
