@@ -1093,8 +1093,9 @@ void poisson_init(cudaStream_t st, const Launch& L, const Geom& g, bool h_loaded
 void sweep(cudaStream_t st, const Launch& L, const Geom& g, const double* hin, double* hout,
            const double* rho, const double* s)
 {
+    const SweepShape sh = sweep_shape(L, g, kSweepThreads64);
     if (15 * g.n < 0x7fffffffLL)
-        sweep_kernel<true><<<L.grid, L.block, 0, st>>>(g, hin, hout, rho, s);
+        sweep_kernel<true><<<sh.grid, sh.block, 0, st>>>(g, hin, hout, rho, s);
     else
         sweep_kernel<false><<<L.grid, L.block, 0, st>>>(g, hin, hout, rho, s);
 }

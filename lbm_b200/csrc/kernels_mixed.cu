@@ -679,9 +679,10 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
         n_normal &= 1;
     }
     const bool off32 = 15 * g.n < 0x7fffffffLL;
+    const SweepShape sh = sweep_shape(L, g, sweep_threads32(g));
     for (int i = 0; i < n_normal; ++i) {
         if (off32)
-            sweep_kernel<<<L.grid, L.block, 0, st>>>(g, mb.h[cur], mb.h[1 - cur], omega, mb.s);
+            sweep_kernel<<<sh.grid, sh.block, 0, st>>>(g, mb.h[cur], mb.h[1 - cur], omega, mb.s);
         else
             sweep_kernel64<<<L.grid, L.block, 0, st>>>(g, mb.h[cur], mb.h[1 - cur], omega, mb.s);
         cur = 1 - cur;
@@ -761,8 +762,9 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
             cur = 1 - cur;
         }
     }
+    const SweepShape sh = sweep_shape(L, g, sweep_threads32(g));
     for (; i < n_normal; ++i) {
-        refine_sweep_kernel<<<L.grid, L.block, 0, st>>>(g, e, mb.h[cur], mb.rr, omega);
+        refine_sweep_kernel<<<sh.grid, sh.block, 0, st>>>(g, e, mb.h[cur], mb.rr, omega);
         e = mb.h[cur];
         cur = 1 - cur;
     }

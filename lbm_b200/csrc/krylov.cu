@@ -273,6 +273,8 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
     const bool border = !kAdj && !g.periodic_x;
     // z run length of the pairs of applications (0: none), as the sweeps'
     const int pair_zlen = !kAdj && m > 3 ? pair_run(g) : 0;
+    // applications without partial sums
+    const SweepShape plain = sweep_shape(L, g, kSweepThreads64);
     double* psum_part = kb.part + 2 * L.nblocks;   // column 2 of the apply kernels' partial sums
     // out = in - A^m in (+ in_d E) (kinds 0, 2) or b_m - (in - A^m in + in_d E)
     // (kind 1), with the kind's partial sums; A^(m-1) in goes through
@@ -286,8 +288,9 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
                 apply2_kernel<<<f2_grid(g, pair_zlen), F2_RC, f2_smem(ApplyOps::kCoefs), st>>>(g, pair_zlen, src, dst, rho);
                 j += 2;
             } else {
-                apply_of<3, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, nullptr, src, dst, rho, nullptr, nullptr, nullptr,
-                                                                   psum_part, L.nblocks, 0.0, border && j == 1, p_ref);
+                const bool sum_p = border && j == 1;
+                apply_of<3, kAdj>(g)<<<sum_p ? L.grid : plain.grid, sum_p ? L.block : plain.block, 0, st>>>(
+                    g, nullptr, src, dst, rho, nullptr, nullptr, nullptr, psum_part, L.nblocks, 0.0, sum_p, p_ref);
                 ++j;
             }
             src = dst;
@@ -325,7 +328,7 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
         const double* cur = kb.w1;
         for (int j = 1; j < m; ++j) {
             double* dst = (j & 1) ? kb.w2 : kb.w1;
-            apply_of<3, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, nullptr, cur, dst, rho, nullptr, nullptr, nullptr,
+            apply_of<3, kAdj>(g)<<<plain.grid, plain.block, 0, st>>>(g, nullptr, cur, dst, rho, nullptr, nullptr, nullptr,
                                                                nullptr, 0, 0.0, 0, 0.0);
             vec_kernel<4><<<kDotBlocks, 256, 0, st>>>(cnt, 0.0, 0.0, kb.bm, nullptr, dst, nullptr, nullptr, nullptr,
                                                        nullptr);

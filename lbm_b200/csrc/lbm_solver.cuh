@@ -107,6 +107,28 @@ inline Launch make_launch(int lx, int ly, int lz, int bx, int by)
     return L;
 }
 
+// Grid and block of a plain sweep (no partial sums): the tile's width and
+// `threads` threads per CTA.  A sweep of a box in L2 is one to three waves of
+// 256-thread CTAs, the last mostly empty; smaller CTAs fill it.  us per sweep,
+// 256 and 32 threads, FP64: 2.70 and 2.41 at 24^3, 2.72 and 2.64 at 32^3, 3.91 and
+// 3.40 at 40^3, 7.89 and 7.50 at 64^3, 14.7 and 13.6 at 72^3, 11.5 and 10.9 at
+// 100x50x64, 84.4 both at 128^3.  FP32 needs 64 warps an SM, so 64 threads (32
+// CTAs at most): 4.82 and 4.60 at 64^3, 4.11 and 3.53 at 24x24x200, 6.98 and 6.65
+// at 100x50x64; below 2^16 cells 128: 24^3 2.00, 1.84 (64) and 1.80 (128), 32^3
+// 2.17, 2.26 and 2.18.
+struct SweepShape {
+    dim3 grid, block;
+};
+inline SweepShape sweep_shape(const Launch& L, const Geom& g, int threads)
+{
+    const int bx = static_cast<int>(L.block.x) < threads ? static_cast<int>(L.block.x) : threads, by = threads / bx;
+    const dim3 grid((g.lx + bx - 1) / bx, (g.ly + by - 1) / by, g.lz);
+    if (grid.y > 65535) return {L.grid, L.block};
+    return {grid, dim3(bx, by, 1)};
+}
+constexpr int kSweepThreads64 = 32;
+inline int sweep_threads32(const Geom& g) { return g.n < (1 << 16) ? 128 : 64; }
+
 // z run length of a two-sweep pass: the grid's waves (tiles x runs over the
 // resident CTAs) times the planes a CTA works through (its run and two halo
 // planes) is least.  *cost: that product.
