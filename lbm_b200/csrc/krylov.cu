@@ -12,7 +12,8 @@
 // consistent (the projected source has zero sum); with the slip walls it is
 // not, and the solve runs on the bordered system of the sweeps' gauged fixed
 // point (bicgstab below).  One iteration is two applications of K
-// (each one pass over the populations, like a sweep) and the vector updates;
+// (each one pass over the populations, like a sweep) and the vector updates
+// (those of p and s within a polynomial's first application);
 // the five inner products per iteration are fixed-order block partial sums
 // added on the host.  The exit: ||b - (I - K) h||_2 < tolerance ||b||_2.
 #include <cuda_runtime.h>
@@ -121,6 +122,52 @@ template <int kKind, bool kAdj>
 auto apply_of(const Geom& g)
 {
     return 15 * g.n < 0x7fffffffLL ? apply_kernel<kKind, kAdj, unsigned> : apply_kernel<kKind, kAdj, long long>;
+}
+
+// A vector update and the first application of the polynomial to its result
+// (forward operator): y = the update, out = K y.  The pull reads every element
+// of y's inputs once, so the thread that pulls an element updates it, in place.
+// kOp 0: y = x0 + a0 (y - a1 x1); kOp 1: y = x0 - a0 x1 (vec_kernel's).  With
+// sum_p the partial sums of apply_kernel's kind 3.  Memory-bound: 5 and 4
+// vectors moved instead of the two launches' 6 and 5; a degree-8 iteration at
+// 128^3 1.80 -> 1.72 ms.
+template <int kOp, class I>
+__global__ void __launch_bounds__(256)
+update_apply_kernel(Geom g, double a0, double a1, double* __restrict__ y, const double* __restrict__ x0,
+                    const double* __restrict__ x1, double* __restrict__ out, const double* __restrict__ rho,
+                    double* __restrict__ part, long long nblocks, int sum_p)
+{
+    int x, yy, z;
+    const bool active = kcell(g, x, yy, z);
+    double p = 0.0;
+    if (active) {
+        const I n = static_cast<I>(g.n);
+        const I c = static_cast<I>(cell_of(g, x, yy, z));
+        const Wrap wr(g, x, yy, z);
+        double hv[Q];
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            const I i = static_cast<I>(q) * n + static_cast<I>(pull_src<q>(g, wr, x, yy, z));
+            if constexpr (kOp == 0) hv[q] = __ldg(x0 + i) + a0 * (y[i] - a1 * __ldg(x1 + i));
+            else hv[q] = __ldg(x0 + i) - a0 * __ldg(x1 + i);
+        });
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            y[static_cast<I>(q) * n + static_cast<I>(pull_src<q>(g, wr, x, yy, z))] = hv[q];
+        });
+        bounce_regs(hv, g, x);
+        static_for<0, Q>([&](auto qc) { p += hv[decltype(qc)::value]; });
+        const double inv_tau = 1.0 / (1.0 / __ldg(rho + c) + 0.5);
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            constexpr double E = wE(q);
+            out[static_cast<I>(q) * n + c] = hv[q] - (hv[q] - E * p) * inv_tau;
+        });
+    }
+    if (sum_p) {
+        double r1[1] = {p};
+        block_sum_store<1>(r1, part, nblocks, block_linear());
+    }
 }
 
 // K twice in one pass (kind 3 twice; forward operator): half the memory traffic
@@ -279,10 +326,12 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
     // out = in - A^m in (+ in_d E) (kinds 0, 2) or b_m - (in - A^m in + in_d E)
     // (kind 1), with the kind's partial sums; A^(m-1) in goes through
     // kb.w1 / kb.w2.  p_ref: subtracted from p in the row's partial sums.
-    auto apply = [&](auto kindc, const double* in, double* out, const double* w, double in_d, double p_ref) {
+    // done: 1 where kb.w1 holds A in already (update_apply).
+    auto apply = [&](auto kindc, const double* in, double* out, const double* w, double in_d, double p_ref,
+                     int done = 0) {
         constexpr int kKind = decltype(kindc)::value;
-        const double* src = in;
-        for (int j = 1; j < m;) {
+        const double* src = done ? kb.w1 : in;
+        for (int j = 1 + done; j < m;) {
             double* dst = src == kb.w1 ? kb.w2 : kb.w1;
             if (j > 1 && j + 1 < m && pair_zlen > 0) {
                 apply2_kernel<<<f2_grid(g, pair_zlen), F2_RC, f2_smem(ApplyOps::kCoefs), st>>>(g, pair_zlen, src, dst, rho);
@@ -298,6 +347,20 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
         apply_of<kKind, kAdj>(g)<<<L.grid, L.block, 0, st>>>(g, in, src, out, rho, s, m > 1 ? kb.bm : nullptr, w,
                                                               kb.part, L.nblocks, border ? in_d : 0.0,
                                                               border && m == 1, p_ref);
+    };
+    // y = the update and A y into kb.w1, returning 1; 0 where the update is a
+    // launch of its own: degree 1, whose one application reads y at its own
+    // cells too, and the adjoint, whose walls read some elements twice
+    auto update_apply = [&](auto opc, double a0, double a1, double* y, const double* x0, const double* x1) -> int {
+        constexpr int kOp = decltype(opc)::value;
+        if (kAdj || m == 1) {
+            vec_kernel<kOp><<<kDotBlocks, 256, 0, st>>>(cnt, a0, a1, y, nullptr, x0, x1, nullptr, nullptr, nullptr);
+            return 0;
+        }
+        auto kern = 15 * g.n < 0x7fffffffLL ? update_apply_kernel<kOp, unsigned> : update_apply_kernel<kOp, long long>;
+        kern<<<border ? L.grid : plain.grid, border ? L.block : plain.block, 0, st>>>(
+            g, a0, a1, y, x0, x1, kb.w1, rho, psum_part, L.nblocks, border);
+        return 1;
     };
     using K0 = std::integral_constant<int, 0>;
     using K1 = std::integral_constant<int, 1>;
@@ -411,15 +474,15 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
             if (budget) break;
             continue;
         }
+        int done = 0;
         if (!first) {
             const double beta = (rho_new / rho_old) * (alpha / omega);
-            vec_kernel<0><<<kDotBlocks, 256, 0, st>>>(cnt, beta, omega, kb.p, nullptr, kb.r, kb.v, nullptr, nullptr,
-                                                       nullptr);
+            done = update_apply(K0{}, beta, omega, kb.p, kb.r, kb.v);
             pd = rd + beta * (pd - omega * vd);
         }
         const bool fresh = first;
         first = false;
-        apply(K0{}, kb.p, kb.v, kb.r0, pd, 0.0);
+        apply(K0{}, kb.p, kb.v, kb.r0, pd, 0.0, done);
         if (!host_sum(L.nblocks, ac, d2)) return LBM_ERR_CUDA;
         if (border) {
             vd = d2[2];
@@ -437,9 +500,9 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
             continue;
         }
         alpha = rho_new / d2[0];
-        vec_kernel<1><<<kDotBlocks, 256, 0, st>>>(cnt, alpha, 0.0, kb.s, nullptr, kb.r, kb.v, nullptr, nullptr, nullptr);
+        done = update_apply(K1{}, alpha, 0.0, kb.s, kb.r, kb.v);
         sd = rd - alpha * vd;
-        apply(K2{}, kb.s, kb.t, kb.s, sd, 0.0);
+        apply(K2{}, kb.s, kb.t, kb.s, sd, 0.0, done);
         if (!host_sum(L.nblocks, ac, d2)) return LBM_ERR_CUDA;
         if (border) {
             td = d2[2];
