@@ -486,13 +486,14 @@ namespace {
 
 // z run length of the two-sweep passes on any box (partial tiles store nothing
 // outside it) and whether they take the tall tile; 0 where single sweeps are
-// faster (*zlen_tall: the tall tile's in any case).  Both sides' times on B200 (us per sweep): a pass takes 0.93 per wave
-// and plane of its CTAs on 32 x 8 tiles (two per SM; 128^3: 29.8 at 34, 256^3:
-// 226 at 238, 141 x 99 x 141: 31.9 at 36) and 0.91 on 32 x 16 (one per SM; 29.1,
-// 223, 34.2 at 38), a single sweep 20.5 per 10^6 cells from DRAM (128^3: 45,
-// 96^3: 18.5, 141 x 99 x 75: 27) and 1.75 + 13 per 10^6 cells while both h
-// buffers stay in L2 (80^3: 8.5, 64^3: 4.9, 32^3: 2.1; 120 B per cell, up to
-// 7.5 * 10^5 cells).
+// faster (*zlen_tall: the tall tile's in any case).  Both sides' times on B200
+// (us per sweep): a pass takes 0.93 per wave and plane of its CTAs on 32 x 8
+// tiles (two per SM; 128^3: 29.8 at 34, 256^3: 226 at 238, 141 x 99 x 141: 31.9
+// at 36) and 0.91 on 32 x 16 (one per SM; 29.1, 223, 34.2 at 38).  A single
+// sweep takes 1.75 + 13 per 10^6 cells while both h buffers stay in L2 (120 B per
+// cell; 80^3: 8.4, 64^3: 4.6, 32^3: 2.1), beyond 5.4 * 10^5 cells 20.5 per 10^6
+// cells less a remainder that stays there (84^3: 11.0, 88^3: 13.0, where the pass
+// takes 11.8), and 20.5 from DRAM (128^3: 45, 96^3: 18.4, 141 x 99 x 75: 27).
 int sweep2_zlen(const Geom& g, int sms, bool* tall, int* zlen_tall)
 {
     auto tiles = [&](int ty) {
@@ -503,7 +504,9 @@ int sweep2_zlen(const Geom& g, int sms, bool* tall, int* zlen_tall)
     const int high = *zlen_tall = two_sweep_zlen(tiles(S2_TALL), g.lz, sms, &tall_cost);
     *tall = tall_cost <= low_cost;
     const double mcells = 1e-6 * static_cast<double>(g.n);
-    const double single = mcells <= 0.75 ? 1.75 + 13.0 * mcells : 20.5 * mcells;
+    const double single = mcells <= 0.54   ? 1.75 + 13.0 * mcells
+                          : mcells <= 0.75 ? 20.5 * mcells - 1.2
+                                           : 20.5 * mcells;
     const double pass = *tall ? 0.91 * static_cast<double>(tall_cost) : 0.93 * static_cast<double>(low_cost);
     return pass < single ? (*tall ? high : low) : 0;
 }
