@@ -432,7 +432,7 @@ const char* lbm_status_string(lbm_status s);
 int lbm_abi_version(void);
 
 /* Self-check of the FP64 kernels' division (a correctly rounded a/b from a
- * reciprocal computed once per divisor, exact_div.cuh) against the IEEE
+ * reciprocal pair computed once per divisor, exact_div.cuh) against the IEEE
  * division on the current device: `samples` pseudo-random operand pairs of
  * the kinds the kernels divide (stencil constants, relaxation times,
  * densities, arbitrary normals); *mismatches = pairs whose bits differ. */
