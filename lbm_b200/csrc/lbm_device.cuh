@@ -219,6 +219,14 @@ __device__ __forceinline__ int ring_plane(int i)
     return base + (i % slots) * 5 + ring_rank(q);
 }
 
+// Address `bytes` beyond p.
+template <class T>
+__device__ __forceinline__ T* at_byte(T* p, unsigned bytes)
+{
+    using C = typename std::conditional<std::is_const<T>::value, const char, char>::type;
+    return reinterpret_cast<T*>(reinterpret_cast<C*>(p) + bytes);
+}
+
 // x slip overwrite of pulled populations (CPU/Inamuro.cpp:589-623).
 template <class T>
 __device__ __forceinline__ void bounce_regs(T (&v)[Q], const Geom& g, int x)
