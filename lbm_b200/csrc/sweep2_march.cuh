@@ -9,9 +9,9 @@
 // z+2 (in flight while the CTA works from the ring), and after a barrier
 // computes sweep k+1 of plane z at its own cell from the ring (lbm_device.cuh); a
 // second barrier frees the slots that the next plane overwrites.  A cell's
-// coefficients are kept beside the ring for sweep k+1.  Coordinates wrap, so the stream and the slip overwrite
-// are those of two single launches for any box.  Cells outside the box
-// (partial tiles) store nothing.  15 n < 2^31 is required (the launchers check).
+// coefficients are kept beside the ring for sweep k+1.  Coordinates wrap, so the
+// stream and the slip overwrite are those of two single launches for any box.
+// Cells outside the box (partial tiles) store nothing.  15 n < 2^31 is required (the launchers check).
 //
 // What bounds it: FP64 latency and the two barriers at 16 warps per SM; 126
 // registers (15 populations in flight and 15 at work) allow no more, and fewer
@@ -20,7 +20,7 @@
 // against 0.65 for single sweeps; other shapes: 32 x 8 tiles with 11 warps in
 // one CTA 0.45, 30 x 14 in one CTA 0.47, 16 x 12 0.47; neighbouring warps
 // joined by named barriers in place of the CTA barriers 0.44; separate warps
-// for the two sweeps 0.47.
+// for the two sweeps 0.47; the rows requested into L2 a plane ahead 0.48.
 #pragma once
 
 #include <cuda_runtime.h>
