@@ -30,6 +30,7 @@
 
 #include "../../include/lbm_b200.h"
 #include "adjoint.hpp"
+#include "capture.hpp"
 #include "handle_internal.hpp"
 #include "lbm_solver.cuh"
 
@@ -163,17 +164,19 @@ lbm_status sweep_segment(lbm_adjoint* a, int yc, const double* rho, const double
     const Launch& L = a->view.L;
     cudaStream_t st = a->view.stream;
     const int ci = a->cfg.check_interval;
-    ADJ_CUDA(a, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    int c = yc;
-    for (int i = 0; i < ci; ++i) {
-        adj::poisson_sweep(st, L, g, i == ci - 1, a->y[c], a->y[1 - c], rho, lp, a->pi_prev, a->part);
-        c = 1 - c;
-    }
-    cudaMemcpyAsync(a->part_host, a->part, 2 * L.nblocks * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaGraph_t graph = nullptr;
-    ADJ_CUDA(a, cudaStreamEndCapture(st, &graph));
+    cudaError_t e = capture_graph(st, &graph, [&] {
+        int c = yc;
+        for (int i = 0; i < ci; ++i) {
+            adj::poisson_sweep(st, L, g, i == ci - 1, a->y[c], a->y[1 - c], rho, lp, a->pi_prev, a->part);
+            c = 1 - c;
+        }
+        return cudaMemcpyAsync(a->part_host, a->part, 2 * L.nblocks * sizeof(double), cudaMemcpyDeviceToHost, st);
+    });
+    if (e != cudaSuccess)
+        return afail(a, e == cudaErrorMemoryAllocation ? LBM_ERR_OOM : LBM_ERR_CUDA,
+                     std::string("sweep graph capture: ") + cudaGetErrorString(e));
     cudaGraphExec_t& ex = a->seg[yc];
-    cudaError_t e = cudaSuccess;
     if (ex) {
         cudaGraphExecUpdateResultInfo info{};
         if (cudaGraphExecUpdate(ex, graph, &info) != cudaSuccess) {

@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "../../include/lbm_b200.h"
+#include "capture.hpp"
 #include "finalize.cuh"
 #include "mixed_cells.cuh"
 #include "phys_host.hpp"
@@ -653,11 +654,11 @@ lbm_status get_segment(lbm_batch* b, int n_normal, cudaGraphExec_t* out)
         return LBM_OK;
     }
     cudaStream_t st = b->stream;
-    BCUDA(b, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    enqueue_segment(b, n_normal, st);
-    cudaMemcpyAsync(b->ctl_host, b->ctl, b->n * sizeof(BCtl), cudaMemcpyDeviceToHost, st);
     cudaGraph_t graph = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(st, &graph);
+    const cudaError_t e = capture_graph(st, &graph, [&] {
+        enqueue_segment(b, n_normal, st);
+        return cudaMemcpyAsync(b->ctl_host, b->ctl, b->n * sizeof(BCtl), cudaMemcpyDeviceToHost, st);
+    });
     if (e != cudaSuccess) return bfail(b, LBM_ERR_CUDA, std::string("segment capture: ") + cudaGetErrorString(e));
     cudaGraphExec_t ex = nullptr;
     const cudaError_t ie = cudaGraphInstantiate(&ex, graph, 0);

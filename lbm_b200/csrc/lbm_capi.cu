@@ -32,6 +32,7 @@
 
 #include "../../include/lbm_b200.h"
 #include "alloc_set.hpp"
+#include "capture.hpp"
 #include "field_stats.cuh"
 #include "handle_internal.hpp"
 #include "lbm_solver.cuh"
@@ -348,11 +349,12 @@ int enqueue_segment(lbm_handle* h, const SegKey& key, cudaStream_t st)
 lbm_status build_segment(lbm_handle* h, const SegKey& key, cudaGraphExec_t* out, int* end_parity)
 {
     cudaStream_t st = h->stream;
-    LBM_CUDA(h, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    const int cur = enqueue_segment(h, key, st);
-    cudaMemcpyAsync(h->ds_host, h->ds, sizeof(DevState), cudaMemcpyDeviceToHost, st);
+    int cur = key.start_parity;
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamEndCapture(st, &graph);
+    cudaError_t e = capture_graph(st, &graph, [&] {
+        cur = enqueue_segment(h, key, st);
+        return cudaMemcpyAsync(h->ds_host, h->ds, sizeof(DevState), cudaMemcpyDeviceToHost, st);
+    });
     if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(out, graph, 0);
     cudaGraphDestroy(graph);
