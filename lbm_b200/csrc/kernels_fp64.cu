@@ -1102,28 +1102,9 @@ void sweep(cudaStream_t st, const Launch& L, const Geom& g, const double* hin, d
 
 bool sweep2_prepare(const Geom& g)
 {
-    return 15 * g.n < 0x7fffffffLL &&
+    return fp64_pass_fits(g.ly, g.n) &&
            cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 f2_smem(SweepOps::kCoefs)) == cudaSuccess;
-}
-
-// Two sweeps per pass where they are faster, from both sides' times on B200
-// (us per sweep): a pass takes 1.12 per wave and plane of its CTAs (128^3: 60
-// at 54, 256^3: 444 at 374, 96^3: 29 at 26, 64^3: 10.6 at 10).  A single sweep
-// takes 2 + 21 per 10^6 cells while both h buffers stay in L2 (64^3: 7.5, 48^3:
-// 4.2, 32^3: 2.6; 240 B per cell), 33.5 per 10^6 cells from 3 to 4.5 * 10^5 cells,
-// where part of them does (80x64x64: 10.5, 72^3: 13.1, 90x66x60: 12.4; the pass
-// 10.7, 12.1, 10.9), and 39 from DRAM (128^3: 84, 90 x 75 x 131: 39).
-int sweep2_zlen(const Geom& g, int sms)
-{
-    const long long tiles = static_cast<long long>((g.lx + F2_TX - 1) / F2_TX) * ((g.ly + F2_TY - 1) / F2_TY);
-    long long cost = 0;
-    const int zlen = two_sweep_zlen(tiles, g.lz, F2_CTAS * sms, &cost);
-    const double mcells = 1e-6 * static_cast<double>(g.n);
-    const double single = mcells <= 0.3    ? 2.0 + 21.0 * mcells
-                          : mcells <= 0.45 ? 33.5 * mcells
-                                           : 39.0 * mcells;
-    return 1.12 * static_cast<double>(cost) < single ? zlen : 0;
 }
 
 void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double* hout,

@@ -188,15 +188,15 @@ sweep_kernel64(Geom g, const float* __restrict__ hin, float* __restrict__ hout,
 // one CTA per 32 x 8 or 32 x 16 tile of output cells and run of `zlen` planes;
 // sweep k on the tile plus its one-cell halo goes into a shared-memory plane
 // ring, sweep k+1 pulls from the ring and only the second result is written.
-// Any box with 15 n < 2^31 (the launcher checks): tiles that reach past it
+// Any box of mixed_pass_fits (the launcher checks): tiles that reach past it
 // store nothing outside.  Bound by instruction issue and load latency at 22 or
 // 20 warps per SM (33 M warp instructions per launch at 128^3, 55 % issue,
 // 0.75 of the HBM rate).  Measured at 256^3 (B200), ms per sweep: 0.222 on 32 x
 // 16 tiles, 0.226 on 32 x 8, 0.235 with one barrier and 45 ring planes; TMA
 // loads of the tiles 0.28 (230 cycles per ten-row box), two cells per thread in
 // packed FP32 pairs 0.235 to 0.28 (as many instructions, fewer warps).
-constexpr int S2_TX = 32, S2_TY = 8;
-constexpr int S2_TALL = 16;   // the tall tile: 640 threads in one CTA per SM, 83 KB (32 x 8: 352 in two, 46 KB each)
+// (The tall tile, S2_TALL: 640 threads in one CTA per SM, 83 KB; 32 x 8: 352 in
+// two, 46 KB each.)
 
 template <int TY, int kCtas>
 __global__ void __launch_bounds__(sweep2_threads(S2_TX, TY), kCtas)
@@ -482,37 +482,6 @@ float* field_f(MixedBuffers& mb, int which)
 
 }  // namespace
 
-namespace {
-
-// z run length of the two-sweep passes on any box (partial tiles store nothing
-// outside it) and whether they take the tall tile; 0 where single sweeps are
-// faster (*zlen_tall: the tall tile's in any case).  Both sides' times on B200
-// (us per sweep): a pass takes 0.93 per wave and plane of its CTAs on 32 x 8
-// tiles (two per SM; 128^3: 29.8 at 34, 256^3: 226 at 238, 141 x 99 x 141: 31.9
-// at 36) and 0.91 on 32 x 16 (one per SM; 29.1, 223, 34.2 at 38).  A single
-// sweep takes 1.75 + 13 per 10^6 cells while both h buffers stay in L2 (120 B per
-// cell; 80^3: 8.4, 64^3: 4.6, 32^3: 2.1), beyond 5.4 * 10^5 cells 20.5 per 10^6
-// cells less a remainder that stays there (84^3: 11.0, 88^3: 13.0, where the pass
-// takes 11.8), and 20.5 from DRAM (128^3: 45, 96^3: 18.4, 141 x 99 x 75: 27).
-int sweep2_zlen(const Geom& g, int sms, bool* tall, int* zlen_tall)
-{
-    auto tiles = [&](int ty) {
-        return static_cast<long long>((g.lx + S2_TX - 1) / S2_TX) * ((g.ly + ty - 1) / ty);
-    };
-    long long low_cost = 0, tall_cost = 0;
-    const int low = two_sweep_zlen(tiles(S2_TY), g.lz, 2LL * sms, &low_cost);
-    const int high = *zlen_tall = two_sweep_zlen(tiles(S2_TALL), g.lz, sms, &tall_cost);
-    *tall = tall_cost <= low_cost;
-    const double mcells = 1e-6 * static_cast<double>(g.n);
-    const double single = mcells <= 0.54   ? 1.75 + 13.0 * mcells
-                          : mcells <= 0.75 ? 20.5 * mcells - 1.2
-                                           : 20.5 * mcells;
-    const double pass = *tall ? 0.91 * static_cast<double>(tall_cost) : 0.93 * static_cast<double>(low_cost);
-    return pass < single ? (*tall ? high : low) : 0;
-}
-
-}  // namespace
-
 lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
 {
     const size_t n = static_cast<size_t>(g.n);
@@ -542,10 +511,13 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             sms = 148;
-        zlen = sweep2_zlen(g, sms, &mb.fuse_tall, &zlen_tall);
+        const MixedPass m = mixed_pass(g.lx, g.ly, g.lz, sms);
+        zlen = m.zlen;
+        zlen_tall = m.zlen_tall;
+        mb.fuse_tall = m.tall;
     }
-    if (zlen > 0 && 15 * g.n < 0x7fffffffLL &&
-        cudaFuncSetAttribute(sweep2_kernel<S2_TALL, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (zlen > 0 && mixed_pass_fits(g.ly, g.n) &&
+        cudaFuncSetAttribute(sweep2_kernel<S2_TALL, S2_TALL_CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess &&
         cudaFuncSetAttribute(sweep2_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess) {
@@ -673,7 +645,7 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
     if (mb.fuse_zlen > 0) {
         const int ty = mb.fuse_tall ? S2_TALL : S2_TY;
         const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + ty - 1) / ty, (g.lz + mb.fuse_zlen - 1) / mb.fuse_zlen);
-        auto kern = mb.fuse_tall ? sweep2_kernel<S2_TALL, 1> : sweep2_kernel<S2_TY, 2>;
+        auto kern = mb.fuse_tall ? sweep2_kernel<S2_TALL, S2_TALL_CTAS> : sweep2_kernel<S2_TY, S2_CTAS>;
         for (int i = 0; i + 1 < n_normal; i += 2) {
             kern<<<grid, sweep2_threads(S2_TX, ty), sweep2_smem(S2_TX, ty), st>>>(g, mb.fuse_zlen, mb.h[cur], mb.h[1 - cur],
                                                                                   omega, mb.s);

@@ -284,7 +284,7 @@ int pair_run(const Geom& g)
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
-    const int zlen = 15 * g.n < 0x7fffffffLL ? fp64::sweep2_zlen(g, sms) : 0;
+    const int zlen = fp64_pass_zlen(g.lx, g.ly, g.lz, sms);
     return zlen > 0 && cudaFuncSetAttribute(apply2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             f2_smem(ApplyOps::kCoefs)) == cudaSuccess
                ? zlen

@@ -1205,7 +1205,7 @@ lbm_status lbm_create(const lbm_params* prm, lbm_precision precision, int device
         // Two sweeps per pass where that is the faster form; LBM_SWEEP2_ZLEN
         // sets the z run length (0: single sweeps).
         const char* env = std::getenv("LBM_SWEEP2_ZLEN");
-        const int zlen = env ? std::atoi(env) : fp64::sweep2_zlen(h->geom, prop.multiProcessorCount);
+        const int zlen = env ? std::atoi(env) : fp64_pass_zlen(prm->lx, prm->ly, prm->lz, prop.multiProcessorCount);
         h->fuse_zlen = (zlen > 0 && fp64::sweep2_prepare(h->geom)) ? zlen : 0;
         // z-marching collide where its tile divides the box (LBM_COLLIDE_ZLEN,
         // 0 disables).

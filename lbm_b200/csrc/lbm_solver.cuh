@@ -7,6 +7,7 @@
 
 #include "../../include/lbm_b200.h"
 #include "lbm_device.cuh"
+#include "sweep_rules.hpp"
 
 namespace lbm {
 
@@ -129,27 +130,6 @@ inline SweepShape sweep_shape(const Launch& L, const Geom& g, int threads)
 constexpr int kSweepThreads64 = 32;
 inline int sweep_threads32(const Geom& g) { return g.n < (1 << 16) ? 128 : 64; }
 
-// z run length of a two-sweep pass: the grid's waves (tiles x runs over the
-// resident CTAs) times the planes a CTA works through (its run and two halo
-// planes) is least.  *cost: that product.
-inline int two_sweep_zlen(long long tiles, int lz, long long slots, long long* cost)
-{
-    int best = 0;
-    long long least = 0;
-    for (int nz = 1; nz <= lz; ++nz) {
-        const int zlen = (lz + nz - 1) / nz;
-        if (zlen > 40 && nz < lz) continue;
-        if (zlen < 4 && best) break;
-        const long long c = (tiles * ((lz + zlen - 1) / zlen) + slots - 1) / slots * (zlen + 2);
-        if (!best || c < least) {
-            best = zlen;
-            least = c;
-        }
-    }
-    if (cost) *cost = least;
-    return best;
-}
-
 // Buffers of one FP64 box.  Populations are q-major SoA: a[q*n + cell].
 struct Fp64Buffers {
     double* f[2];       // post-collision f* ping-pong
@@ -185,10 +165,8 @@ void poisson_init(cudaStream_t st, const Launch& L, const Geom& g, bool h_loaded
 void sweep(cudaStream_t st, const Launch& L, const Geom& g, const double* hin, double* hout,
            const double* rho, const double* s);
 // Two sweeps per launch (temporal blocking).  sweep2_prepare: whether the box
-// admits it (15 n < 2^31) and the kernel is set up; sweep2_zlen: the z run
-// length for the box on `sms` SMs, 0 where single sweeps are faster.
+// admits it (fp64_pass_fits) and the kernel is set up.
 bool sweep2_prepare(const Geom& g);
-int sweep2_zlen(const Geom& g, int sms);
 void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double* hout,
             const double* rho, const double* s);
 void sweep_check_a(cudaStream_t st, const Launch& L, const Geom& g, const double* hin,

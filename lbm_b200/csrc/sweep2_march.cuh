@@ -11,7 +11,7 @@
 // second barrier frees the slots that the next plane overwrites.  A cell's
 // coefficients are kept beside the ring for sweep k+1.  Coordinates wrap, so the
 // stream and the slip overwrite are those of two single launches for any box.
-// Cells outside the box (partial tiles) store nothing.  15 n < 2^31 is required (the launchers check).
+// Cells outside the box (partial tiles) store nothing.  fp64_pass_fits is required (the launchers check).
 //
 // What bounds it: FP64 latency and the two barriers at 16 warps per SM; 126
 // registers (15 populations in flight and 15 at work) allow no more, and fewer
@@ -26,14 +26,13 @@
 #include <cuda_runtime.h>
 
 #include "lbm_device.cuh"
+#include "sweep_rules.hpp"
 
 namespace lbm {
 
-constexpr int F2_RX = 32, F2_RY = 8;                     // region: tile and halo
-constexpr int F2_TX = F2_RX - 2, F2_TY = F2_RY - 2;      // tile
+constexpr int F2_RX = F2_TX + 2, F2_RY = F2_TY + 2;      // region: tile and halo
 constexpr int F2_RC = F2_RX * F2_RY;
 constexpr int F2_PLANES = ring_planes();
-constexpr int F2_CTAS = 2;                               // per SM
 // Shared memory with `coefs` coefficients per cell (73,728 B with 3).
 constexpr int f2_smem(int coefs) { return (F2_PLANES + 2 * coefs) * F2_RC * static_cast<int>(sizeof(double)); }
 
