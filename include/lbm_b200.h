@@ -431,11 +431,13 @@ const char* lbm_last_error(const lbm_handle* h);
 const char* lbm_status_string(lbm_status s);
 int lbm_abi_version(void);
 
-/* Self-check of the FP64 kernels' division (a correctly rounded a/b from a
- * reciprocal pair computed once per divisor, exact_div.cuh) against the IEEE
- * division on the current device: `samples` pseudo-random operand pairs of
- * the kinds the kernels divide (stencil constants, relaxation times,
- * densities, arbitrary normals); *mismatches = pairs whose bits differ. */
+/* Self-check of the FP64 kernels' division (a/b from a reciprocal pair computed
+ * once per divisor, exact_div.cuh: within 0.5 + 2^-51 ulp for normal finite
+ * operands and quotients, so the correctly rounded quotient unless a/b is within
+ * 2^-104 of a midpoint of two doubles) against the IEEE division on the current
+ * device: `samples` pseudo-random operand pairs of the kinds the kernels divide
+ * (stencil constants, relaxation times, densities, arbitrary normals; every 256th
+ * numerator infinite); *mismatches = pairs whose bits differ. */
 lbm_status lbm_selftest_division(uint64_t samples, uint64_t seed, uint64_t* mismatches);
 
 /* ---- batched boxes ------------------------------------------------------

@@ -18,7 +18,9 @@
 // with a probability of 2^-50; lbm_selftest_division (selftest.cu) finds no
 // difference from CUDA's IEEE division on 2^32 operand pairs.  Where a lo
 // falls below the normal range (|a/b| < 2^-916) it adds at most half an ulp.
-// Divisors must be normal and finite.
+// Divisors must be normal and finite.  A numerator of -0 may give +0 (where lo is
+// negative).  For infinite numerators lo has to have hi's sign, else a hi + a lo is
+// inf - inf or inf * 0: recip_for.
 //
 // Two operations per quotient instead of the two range comparisons and five
 // operations of a remainder-corrected division matter in the two-sweep pass,
@@ -43,6 +45,15 @@ __device__ __forceinline__ RecipPair recip_pair(double b)
     r.hi = __ddiv_rn(1.0, b);
     r.lo = recip_lo(b, r.hi);
     return r;
+}
+
+// The pair for a collision's numerators h - E p.  Where p is not finite (the sum
+// of the cell's h, so wherever one of them is not) they are infinite or NaN, and
+// hi in lo's place gives the IEEE division's quotient, an infinity of the right
+// sign or NaN.
+__device__ __forceinline__ RecipPair recip_for(const RecipPair& r, double p)
+{
+    return {r.hi, (__double2hiint(p) & 0x7ff00000) == 0x7ff00000 ? r.hi : r.lo};
 }
 
 __device__ __forceinline__ double div_rn(double a, const RecipPair& r) { return __fma_rn(a, r.hi, __dmul_rn(a, r.lo)); }

@@ -412,7 +412,7 @@ poisson_init_kernel(Geom g, int h_loaded, const double* __restrict__ hload,
     const long long c = cell_of(g, x, y, z);
     const double pv = p[c];
     const double tauh = 1.0 / rho[c] + 0.5;
-    const RecipPair rt = recip_pair(tauh);
+    const RecipPair rt = recip_for(recip_pair(tauh), pv);
     const double sv = s[c];
     static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
@@ -432,7 +432,7 @@ template <int q>
 __device__ __forceinline__ double collide_h(double h, double pv, const RecipPair& rt, double sv)
 {
     constexpr double E = wE(q);
-    return h - div_rn(h - E * pv, rt) - (E / 3.0) * sv;
+    return h - div_rn(h - E * pv, recip_for(rt, pv)) - (E / 3.0) * sv;
 }
 
 // I: index type (long long in general, int where 15 n < 2^31).

@@ -1,6 +1,7 @@
 // selftest.cu -- lbm_selftest_division: the FP64 kernels' division from
 // a reciprocal pair (exact_div.cuh) against CUDA's IEEE division on
-// pseudo-random operands of the kinds the kernels use.
+// pseudo-random operands of the kinds the kernels use, infinite numerators
+// among them.
 #include <cuda_runtime.h>
 
 #include "../../include/lbm_b200.h"
@@ -35,7 +36,9 @@ __global__ void division_selftest_kernel(unsigned long long n, unsigned long lon
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         const unsigned long long r1 = mix64(seed ^ (2 * i)), r2 = mix64(seed ^ (2 * i + 1));
-        const double a = random_double(r1, -320, 320, true);
+        // (every 256th numerator infinite, as where a cell's p is)
+        const double p = i % 256 ? 0.0 : copysign(HUGE_VAL, random_double(r1, 0, 0, true));
+        const double a = random_double(r1, -320, 320, true) + p;
         double b;
         switch (r2 & 7) {
         case 0: b = 10.0; break;
@@ -45,7 +48,7 @@ __global__ void division_selftest_kernel(unsigned long long n, unsigned long lon
         case 4: b = random_double(r2, -10, 10, false); break;      // densities
         default: b = random_double(r2, -200, 200, true); break;   // any normal divisor
         }
-        const double q = lbm::div_rn(a, lbm::recip_pair(b));
+        const double q = lbm::div_rn(a, lbm::recip_for(lbm::recip_pair(b), p));
         const double ref = __ddiv_rn(a, b);
         if (__double_as_longlong(q) != __double_as_longlong(ref)) ++bad;
     }
