@@ -72,7 +72,8 @@ struct lbm_adjoint {
     size_t part_len = 0;
     double forward_ms = 0.0;
     uint64_t forward_sweeps = 0;
-    cudaGraphExec_t seg[2] = {};        // a check interval of transposed sweeps from y[0] and from y[1]
+    cudaGraphExec_t seg[2] = {};        // a check interval's last transposed sweeps from y[0] and from y[1]
+    cudaGraphExec_t part_seg[2] = {};   // kGraphSweeps of the sweeps ahead of them (intervals longer than that)
     int y_warm = -1;                    // y buffer holding the last converged adjoint iterate, -1: none
     std::vector<double*> bslot;         // binomial mode: checkpoint slots (state_bytes each), allocated on first use
     std::vector<int> bfree;             // free slot indices
@@ -126,9 +127,9 @@ void free_all(lbm_adjoint* a)
                       a->scratch, a->ls, a->lsrc, a->lkf, a->part};
     for (double* p : bufs) cudaFree(p);
     if (a->part_host) cudaFreeHost(a->part_host);
-    for (cudaGraphExec_t& e : a->seg) {
-        if (e) cudaGraphExecDestroy(e);
-        e = nullptr;
+    for (cudaGraphExec_t* e : {&a->seg[0], &a->seg[1], &a->part_seg[0], &a->part_seg[1]}) {
+        if (*e) cudaGraphExecDestroy(*e);
+        *e = nullptr;
     }
     if (a->fwd) lbm_destroy(a->fwd);
 }
@@ -153,30 +154,35 @@ namespace {
 
 double* slot(double* base, long long n, int i) { return base + static_cast<long long>(i) * n; }
 
-// A check interval of transposed sweeps starting from y[yc] (rho, lam p: the
-// step's) and the copy of its partial sums, as one graph: launched one by one
-// the sweeps of a small box wait for the host (32^3: 5.1 us per sweep, 4.4 at
-// 24^3).  A step's pointers differ from the last one's, so the graph of the
-// same shape is captured anew and the executable updated.
-lbm_status sweep_segment(lbm_adjoint* a, int yc, const double* rho, const double* lp)
+// Most sweeps of one graph; even, so that whole graphs return to their iterate.
+// A node takes some 6 KB of the host's memory: an interval of 100 000 sweeps as
+// one graph 580 MB and, on its first pass, 772 ms where launches took 552.
+constexpr int kGraphSweeps = 512;
+
+// `sweeps` transposed sweeps starting from y[yc] (rho, lam p: the step's) as one
+// graph, the last with the check's partial sums and their copy where `check`:
+// launched one by one the sweeps of a small box wait for the host (32^3: 5.1 us
+// per sweep, 4.4 at 24^3).  A step's pointers differ from the last one's, so the
+// graph of the same shape is captured anew and the executable updated.
+lbm_status sweep_segment(lbm_adjoint* a, int yc, int sweeps, bool check, const double* rho, const double* lp,
+                         cudaGraphExec_t& ex)
 {
     const Geom& g = a->view.geom;
     const Launch& L = a->view.L;
     cudaStream_t st = a->view.stream;
-    const int ci = a->cfg.check_interval;
     cudaGraph_t graph = nullptr;
     cudaError_t e = capture_graph(st, &graph, [&] {
         int c = yc;
-        for (int i = 0; i < ci; ++i) {
-            adj::poisson_sweep(st, L, g, i == ci - 1, a->y[c], a->y[1 - c], rho, lp, a->pi_prev, a->part);
+        for (int i = 0; i < sweeps; ++i) {
+            adj::poisson_sweep(st, L, g, check && i == sweeps - 1, a->y[c], a->y[1 - c], rho, lp, a->pi_prev, a->part);
             c = 1 - c;
         }
-        return cudaMemcpyAsync(a->part_host, a->part, 2 * L.nblocks * sizeof(double), cudaMemcpyDeviceToHost, st);
+        return check ? cudaMemcpyAsync(a->part_host, a->part, 2 * L.nblocks * sizeof(double), cudaMemcpyDeviceToHost, st)
+                     : cudaSuccess;
     });
     if (e != cudaSuccess)
         return afail(a, e == cudaErrorMemoryAllocation ? LBM_ERR_OOM : LBM_ERR_CUDA,
                      std::string("sweep graph capture: ") + cudaGetErrorString(e));
-    cudaGraphExec_t& ex = a->seg[yc];
     if (ex) {
         cudaGraphExecUpdateResultInfo info{};
         if (cudaGraphExecUpdate(ex, graph, &info) != cudaSuccess) {
@@ -239,13 +245,16 @@ lbm_status step_adjoint(lbm_adjoint* a, bool first, double* const xn, double* co
     }
     adj::poisson_pi(st, L, g, a->y[yc], a->pi_prev);
     const int ci = a->cfg.check_interval;
+    const int parts = (ci - 1) / kGraphSweeps, last = ci - parts * kGraphSweeps;
     bool captured[2] = {false, false};
     for (; !a->cfg.krylov;) {
         if (!captured[yc]) {
-            s = sweep_segment(a, yc, X1(1), LM(5));
+            s = sweep_segment(a, yc, last, true, X1(1), LM(5), a->seg[yc]);
+            if (s == LBM_OK && parts > 0) s = sweep_segment(a, yc, kGraphSweeps, false, X1(1), LM(5), a->part_seg[yc]);
             if (s != LBM_OK) return s;
             captured[yc] = true;
         }
+        for (int i = 0; i < parts; ++i) ADJ_CUDA(a, cudaGraphLaunch(a->part_seg[yc], st));
         ADJ_CUDA(a, cudaGraphLaunch(a->seg[yc], st));
         if (ci & 1) yc = 1 - yc;
         it += static_cast<uint64_t>(ci);
