@@ -460,7 +460,7 @@ typedef struct {
     int zrun;                /* z planes per work item */
     int ctas_per_sm;         /* persistent grid: ctas_per_sm CTAs per SM */
     int sweep2_zrun;         /* > 0: plain sweeps run two per launch (temporal blocking,
-                                32 x 8 tiles) on z runs of at most this length; 0: one per launch */
+                                32 x 8 or 16 x 8 tiles) on z runs of at most this length; 0: one per launch */
     int reserved;
     double sweep_ms;         /* measured time per sweep of the chosen form (lbm_batch_tune), else 0 */
 } lbm_batch_tuning;

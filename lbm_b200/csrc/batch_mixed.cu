@@ -186,21 +186,25 @@ b_sweep(const BItem* __restrict__ items, int n_items, const BInst* __restrict__ 
     }
 }
 
-// Two-sweep passes: 32 x 8 tiles, two CTAs an SM.  us per sweep of ten boxes of
-// 48 to 96 cells a side (3.77 million cells), all, five and two of them in their
-// loops: 60.9, 31.3, 16.6, against 66.3, 33.9, 17.7 with 16 x 16 tiles, 67.7, 34.2,
-// 16.1 with 16 x 8 (four CTAs), 61.4, 33.0, 16.7 with 32 x 16 (one CTA) and 70 to
-// 76 with 30 x 8, 30 x 14, 16 x 32 and 14 x 14.
-constexpr int B2_TX = 32, B2_TY = 8;
-constexpr int B2_THREADS = sweep2_threads(B2_TX, B2_TY);   // 352
-constexpr int B2_SMEM = sweep2_smem(B2_TX, B2_TY);         // 46,240 B
-constexpr int B2_CTAS_PER_SM = 2;
+// Tiles of the two-sweep passes: 32 x 8 recomputes fewer halo cells, 16 x 8 wastes
+// fewer cells past the end of a row.  A batch takes 16 x 8 where 32 x 8 covers more
+// than 1.17 times the cells (pick_tile2).  us per sweep of ten boxes, all in their
+// loops, 32 x 8 and 16 x 8: 64^3 42.0 and 46.6, 32^3 (64 boxes) 33.3 and 34.7, two of
+// 96^3 26.7 and 29.8 (1.0 times the cells); 98^3 (four) 72.9 and 73.1, 112x64x48 48.6
+// and 49.0 (1.14); 80^3 (five) 49.7 and 44.2, 66x50x70 (six) 33.1 and 31.7 (1.2); 48^3
+// 24.6 and 19.6, 33^3 16.5 and 13.0, 36x40x64 27.3 and 23.0 (1.33); 16x48x96 23.1 and
+// 13.6 (2).  16 x 16, 32 x 16, 30 x 8, 30 x 14, 16 x 32 and 14 x 14 were no better than
+// these on boxes of 48 to 96 cells a side.
+struct Tile2 {
+    int tx, ty, ctas;   // cells, resident CTAs per SM
+};
+constexpr Tile2 kTile2[2] = {{32, 8, 2}, {16, 8, 4}};   // 352 threads, 46,240 B; 192 threads, 24,480 B
 constexpr int kPlanRuns = 64;      // longest run (sweep2_zrun's limit)
 constexpr int kPlanShortest = 4;   // shortest, unless sweep2_zrun is below it
 
-__device__ __forceinline__ int b2_tiles(const Geom& g)
+__host__ __device__ __forceinline__ int tiles2(const Geom& g, int tx, int ty)
 {
-    return ((g.lx + B2_TX - 1) / B2_TX) * ((g.ly + B2_TY - 1) / B2_TY);
+    return ((g.lx + tx - 1) / tx) * ((g.ly + ty - 1) / ty);
 }
 
 // Work list of the two-sweep passes of a segment, rebuilt before it: the items
@@ -213,7 +217,7 @@ __device__ __forceinline__ int b2_tiles(const Geom& g)
 // segment).  With a fixed list whose items of instances that have left are
 // skipped: 38.5 us per sweep with five of the ten boxes left and 23.4 with two.
 __global__ void __launch_bounds__(256)
-b_plan2(const BInst* __restrict__ inst, const BCtl* __restrict__ ctl, int n, int zmax, int slots,
+b_plan2(const BInst* __restrict__ inst, const BCtl* __restrict__ ctl, int n, int tx, int ty, int zmax, int slots,
         BItem* __restrict__ items, int* __restrict__ n_items)
 {
     __shared__ int total[kPlanRuns + 1];
@@ -226,7 +230,7 @@ b_plan2(const BInst* __restrict__ inst, const BCtl* __restrict__ ctl, int n, int
     const int z = threadIdx.x % kPlanRuns + 1;
     int mine = 0;
     for (int i = threadIdx.x / kPlanRuns; i < n; i += 256 / kPlanRuns)
-        if (ctl[i].active) mine += b2_tiles(inst[i].g) * ((inst[i].g.lz + z - 1) / z);
+        if (ctl[i].active) mine += tiles2(inst[i].g, tx, ty) * ((inst[i].g.lz + z - 1) / z);
     atomicAdd(&total[z], mine);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -243,24 +247,25 @@ b_plan2(const BInst* __restrict__ inst, const BCtl* __restrict__ ctl, int n, int
     __syncthreads();
     int before = 0;
     for (int i = threadIdx.x; i < me; i += blockDim.x)
-        if (ctl[i].active) before += b2_tiles(inst[i].g) * ((inst[i].g.lz + best - 1) / best);
+        if (ctl[i].active) before += tiles2(inst[i].g, tx, ty) * ((inst[i].g.lz + best - 1) / best);
     atomicAdd(&first, before);
     __syncthreads();
     if (me == 0 && threadIdx.x == 0) *n_items = total[best];
     if (!ctl[me].active) return;
     const Geom g = inst[me].g;
-    const int nx = (g.lx + B2_TX - 1) / B2_TX, per = b2_tiles(g);
+    const int nx = (g.lx + tx - 1) / tx, per = tiles2(g, tx, ty);
     // (len <= best, so that (nz - 1) len < lz: no run is empty)
     const int nz = (g.lz + best - 1) / best, len = (g.lz + nz - 1) / nz;
     for (int k = threadIdx.x; k < per * nz; k += blockDim.x) {
         const int r = k % per, z0 = k / per * len;
-        items[first + k] = BItem{me, r % nx * B2_TX, r / nx * B2_TY, z0, min(z0 + len, g.lz)};
+        items[first + k] = BItem{me, r % nx * tx, r / nx * ty, z0, min(z0 + len, g.lz)};
     }
 }
 
 // Two plain sweeps (flip index j: state in h[(parity + j) & 1], result in the
 // other buffer) for every item of the plan, with temporal blocking (sweep2_run).
-__global__ void __launch_bounds__(B2_THREADS, B2_CTAS_PER_SM)
+template <int kTile>
+__global__ void __launch_bounds__(sweep2_threads(kTile2[kTile].tx, kTile2[kTile].ty), kTile2[kTile].ctas)
 b_sweep2(const BItem* __restrict__ items, const int* __restrict__ n_items, const BInst* __restrict__ inst,
          const BCtl* __restrict__ ctl, int j, BPool B)
 {
@@ -272,7 +277,7 @@ b_sweep2(const BItem* __restrict__ items, const int* __restrict__ n_items, const
         const bool odd = ((ctl[w.inst].parity + j) & 1) != 0;
         const float* hin = (odd ? B.h[1] : B.h[0]) + I.pop;
         float* hout = (odd ? B.h[0] : B.h[1]) + I.pop;
-        sweep2_run<B2_TX, B2_TY>(I.g, w.x0, w.y0, w.z0, w.z1, hin, hout, B.omega + I.fld, B.s + I.fld, ring);
+        sweep2_run<kTile2[kTile].tx, kTile2[kTile].ty>(I.g, w.x0, w.y0, w.z0, w.z1, hin, hout, B.omega + I.fld, B.s + I.fld, ring);
         __syncthreads();   // the ring is reused by the CTA's next item
     }
 }
@@ -447,6 +452,7 @@ struct lbm_batch {
     long long pop_elems = 0;         // elements of one pooled population buffer
     long long item_capacity = 0;     // partial-sum slots allocated (largest work list of any tuning)
     int n_items = 0;
+    int tile2 = 0;                   // tile of the two-sweep passes (kTile2)
     int* n_items2_d = nullptr;       // two-sweep work list of the running segment (b_plan2)
     BInst* inst_d = nullptr;
     BItem* items_d = nullptr;
@@ -501,6 +507,15 @@ long long count_items(const std::vector<lbm_params>& prm, int tx, int ty, int zr
     for (const auto& p : prm)
         c += static_cast<long long>((p.lx + tx - 1) / tx) * ((p.ly + ty - 1) / ty) * ((p.lz + zrun - 1) / zrun);
     return c;
+}
+
+// Tile of the two-sweep passes for these boxes (kTile2).
+int pick_tile2(const std::vector<lbm_params>& prm)
+{
+    double covered[2];
+    for (int t = 0; t < 2; ++t)
+        covered[t] = static_cast<double>(count_items(prm, kTile2[t].tx, kTile2[t].ty, 1)) * kTile2[t].tx * kTile2[t].ty;
+    return covered[0] > 1.17 * covered[1] ? 1 : 0;
 }
 
 // Rebuilds the work list for the batch's tuning (instance-major items).
@@ -609,17 +624,21 @@ lbm_status load_instance(lbm_batch* b, int i, const double* const src[6])
 }
 
 // The two-sweep passes' work list for the segment to come, and one pass.
-int grid2_of(const lbm_batch* b) { return B2_CTAS_PER_SM * b->sm_count; }
+int grid2_of(const lbm_batch* b) { return kTile2[b->tile2].ctas * b->sm_count; }
 
 void enqueue_plan2(lbm_batch* b, cudaStream_t st)
 {
-    b_plan2<<<b->n, 256, 0, st>>>(b->inst_d, b->ctl, b->n, b->tune.sweep2_zrun, grid2_of(b), b->items2_d,
+    const Tile2& t = kTile2[b->tile2];
+    b_plan2<<<b->n, 256, 0, st>>>(b->inst_d, b->ctl, b->n, t.tx, t.ty, b->tune.sweep2_zrun, grid2_of(b), b->items2_d,
                                   b->n_items2_d);
 }
 
 void enqueue_sweep2(lbm_batch* b, int j, cudaStream_t st)
 {
-    b_sweep2<<<grid2_of(b), B2_THREADS, B2_SMEM, st>>>(b->items2_d, b->n_items2_d, b->inst_d, b->ctl, j, b->pool);
+    const Tile2& t = kTile2[b->tile2];
+    auto kern = b->tile2 == 0 ? b_sweep2<0> : b_sweep2<1>;
+    kern<<<grid2_of(b), sweep2_threads(t.tx, t.ty), sweep2_smem(t.tx, t.ty), st>>>(b->items2_d, b->n_items2_d, b->inst_d,
+                                                                                  b->ctl, j, b->pool);
 }
 
 // One segment's kernels on st (a capturing stream): n_normal plain sweeps
@@ -962,7 +981,7 @@ lbm_status lbm_batch_create(const lbm_params* params, int n_instances, int devic
     const long long cap = b->item_capacity;
     ok = ok && okd(&b->part_src, 3 * cap) && okd(&b->part_mass, cap) && okd(&b->part_prep, 3 * cap) &&
          okd(&b->part_a, cap) && okd(&b->part_b, 5 * cap);
-    ok = ok && cudaMalloc(&b->items2_d, count_items(b->prm, B2_TX, B2_TY, 1) * sizeof(BItem)) == cudaSuccess &&
+    ok = ok && cudaMalloc(&b->items2_d, count_items(b->prm, kTile2[1].tx, kTile2[1].ty, 1) * sizeof(BItem)) == cudaSuccess &&
          cudaMalloc(&b->n_items2_d, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMalloc(&b->inst_d, n_instances * sizeof(BInst)) == cudaSuccess &&
          cudaMalloc(&b->ds, n_instances * sizeof(DevState)) == cudaSuccess &&
@@ -977,6 +996,7 @@ lbm_status lbm_batch_create(const lbm_params* params, int n_instances, int devic
     }
     cudaMemset(b->pool.s, 0, fld * sizeof(float));
     cudaMemset(b->pool.omega, 0, fld * sizeof(float));
+    b->tile2 = pick_tile2(b->prm);
     if (const char* e = std::getenv("LBM_BATCH_TUNING")) {
         lbm_batch_tuning t{};
         const int got = std::sscanf(e, "%d,%d,%d,%d,%d", &t.tile_x, &t.tile_y, &t.zrun, &t.ctas_per_sm,
@@ -1104,7 +1124,32 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
     const int ctas[3] = {2, 4, 8};
     lbm_batch_tuning best = b->tune;
     best.sweep_ms = 1e30;
+    // A form's time per launch, in a graph as the segments are (launched one by one
+    // the sweeps of small boxes wait for the host, single sweeps the longest).
     const int reps = 6;
+    auto time_launches = [&](int launches, auto&& launch, double* ms_each) -> lbm_status {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t ex = nullptr;
+        cudaError_t e = capture_graph(st, &graph, [&] {
+            for (int r = 0; r < launches; ++r) launch(r);
+            return cudaSuccess;
+        });
+        BCUDA(b, e);
+        e = cudaGraphInstantiate(&ex, graph, 0);
+        cudaGraphDestroy(graph);
+        BCUDA(b, e);
+        e = cudaGraphLaunch(ex, st);
+        if (e == cudaSuccess) e = cudaEventRecord(b->ev[0], st);
+        if (e == cudaSuccess) e = cudaGraphLaunch(ex, st);
+        if (e == cudaSuccess) e = cudaEventRecord(b->ev[1], st);
+        if (e == cudaSuccess) e = cudaEventSynchronize(b->ev[1]);
+        float ms = 0.f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
+        cudaGraphExecDestroy(ex);
+        BCUDA(b, e);
+        *ms_each = ms / launches;
+        return LBM_OK;
+    };
     for (auto& tl : tiles)
         for (int zr : zruns)
             for (int cp : ctas) {
@@ -1113,19 +1158,14 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
                 lbm_status s = build_items(b);
                 if (s != LBM_OK) return s;
                 const int grid = grid_of(b);
-                for (int r = 0; r < 2; ++r)
+                double ms = 0.0;
+                s = time_launches(reps, [&](int r) {
                     b_sweep<<<grid, 256, 0, st>>>(b->items_d, b->n_items, b->inst_d, t.tile_x, b->ctl, r, b->pool);
-                BCUDA(b, cudaEventRecord(b->ev[0], st));
-                for (int r = 0; r < reps; ++r)
-                    b_sweep<<<grid, 256, 0, st>>>(b->items_d, b->n_items, b->inst_d, t.tile_x, b->ctl, r, b->pool);
-                BCUDA(b, cudaEventRecord(b->ev[1], st));
-                BCUDA(b, cudaGetLastError());
-                BCUDA(b, cudaEventSynchronize(b->ev[1]));
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
-                if (ms / reps < best.sweep_ms) {
+                }, &ms);
+                if (s != LBM_OK) return s;
+                if (ms < best.sweep_ms) {
                     best = t;
-                    best.sweep_ms = ms / reps;
+                    best.sweep_ms = ms;
                 }
             }
     // two sweeps per launch on z runs of 8, 16, 32 (per-sweep time = launch / 2)
@@ -1138,18 +1178,12 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
         lbm_status s = build_items(b);
         if (s != LBM_OK) return s;
         enqueue_plan2(b, st);
-        enqueue_sweep2(b, 0, st);
-        BCUDA(b, cudaEventRecord(b->ev[0], st));
-        for (int r = 0; r < reps / 2; ++r) enqueue_sweep2(b, r, st);
-        BCUDA(b, cudaEventRecord(b->ev[1], st));
-        BCUDA(b, cudaGetLastError());
-        BCUDA(b, cudaEventSynchronize(b->ev[1]));
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
-        const double per_sweep = ms / (reps / 2) / 2.0;
-        if (per_sweep < best.sweep_ms) {
+        double ms = 0.0;
+        s = time_launches(reps / 2, [&](int r) { enqueue_sweep2(b, r, st); }, &ms);
+        if (s != LBM_OK) return s;
+        if (ms / 2.0 < best.sweep_ms) {
             best = t;
-            best.sweep_ms = per_sweep;
+            best.sweep_ms = ms / 2.0;
         }
     }
     b->tune = best;
