@@ -14,6 +14,7 @@ solver call raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 import os
 import re
@@ -246,7 +247,27 @@ def _dp(a: np.ndarray):
 
 
 _HUGE_PAGE = 1 << 21
-_libc = C.CDLL(None)
+
+
+@functools.lru_cache(maxsize=None)
+def _page_allocator():
+    """(set, handler): NumPy's PyDataMem_SetHandler and the allocator of
+    host_pages.cpp as its argument; None where NumPy has no such thing."""
+    try:
+        from numpy._core import _multiarray_umath as core
+    except ImportError:
+        from numpy.core import _multiarray_umath as core
+    if not hasattr(core, "get_handler_name"):
+        return None
+    pointer = C.pythonapi.PyCapsule_GetPointer
+    pointer.restype, pointer.argtypes = C.c_void_p, [C.py_object, C.c_char_p]
+    capsule = C.pythonapi.PyCapsule_New
+    capsule.restype, capsule.argtypes = C.py_object, [C.c_void_p, C.c_char_p, C.c_void_p]
+    api = C.cast(pointer(core._ARRAY_API, None), C.POINTER(C.c_void_p))
+    set_handler = C.PYFUNCTYPE(C.py_object, C.py_object)(api[304])   # its slot in NumPy's C API since 1.22
+    table = load_library().lbm_host_pages
+    table.restype = C.c_void_p
+    return set_handler, capsule(table(), b"mem_handler", None)
 
 
 def _host_array(shape) -> np.ndarray:
@@ -255,13 +276,15 @@ def _host_array(shape) -> np.ndarray:
     costs more than the copy (64 of 84 ms for sixty arrays of 2 to 4 MB); numpy
     asks for huge pages from 4 MB on, and a plain allocation seldom holds one
     of 2 MB whole, so the array starts on a huge page.  48 ms so."""
-    size = 8 * math.prod(shape)
-    if size < _HUGE_PAGE:
+    got = _page_allocator() if 8 * math.prod(shape) >= _HUGE_PAGE else None
+    if got is None:
         return np.empty(shape)
-    raw = np.empty(size + _HUGE_PAGE, np.uint8)
-    first = -raw.ctypes.data % _HUGE_PAGE
-    _libc.madvise(C.c_void_p(raw.ctypes.data + first), C.c_size_t(size // _HUGE_PAGE * _HUGE_PAGE), C.c_int(14))
-    return raw[first:first + size].view(np.float64).reshape(shape)
+    set_handler, handler = got
+    before = set_handler(handler)   # (of this context alone: other threads keep theirs)
+    try:
+        return np.empty(shape)
+    finally:
+        set_handler(before)
 
 
 def params_default() -> Params:
