@@ -503,9 +503,10 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
     mb.dwz = nullptr;
     mb.fuse_zlen = 0;
     mb.fuse_tall = false;
-    int zlen = 0, zlen_tall = 0;
+    mb.refine_zlen = 0;
+    int zlen = 0, refine_zlen = 0;
     if (const char* env = std::getenv("LBM_SWEEP2_ZLEN")) {
-        zlen = zlen_tall = std::atoi(env);
+        zlen = refine_zlen = std::atoi(env);
     } else {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -513,16 +514,16 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
             sms = 148;
         const MixedPass m = mixed_pass(g.lx, g.ly, g.lz, sms);
         zlen = m.zlen;
-        zlen_tall = m.zlen_tall;
+        refine_zlen = m.refine_zlen;
         mb.fuse_tall = m.tall;
     }
-    if (zlen > 0 && mixed_pass_fits(g.ly, g.n) &&
+    if ((zlen > 0 || refine_zlen > 0) && mixed_pass_fits(g.ly, g.n) &&
         cudaFuncSetAttribute(sweep2_kernel<S2_TALL, S2_TALL_CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess &&
         cudaFuncSetAttribute(sweep2_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess) {
-        mb.fuse_zlen = zlen;
-        mb.refine_zlen = zlen_tall;
+        mb.fuse_zlen = zlen > 0 ? zlen : 0;
+        mb.refine_zlen = refine_zlen > 0 ? refine_zlen : 0;
     }
     // z-marching collide where its tile divides the box.
     const char* cenv = std::getenv("LBM_COLLIDE_ZLEN");
@@ -727,7 +728,7 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
     const float* e = mb.rr;
     int cur = 0;
     int i = 1;
-    if (mb.fuse_zlen > 0) {
+    if (mb.refine_zlen > 0) {
         const dim3 grid((g.lx + S2_TX - 1) / S2_TX, (g.ly + S2_TALL - 1) / S2_TALL,
                         (g.lz + mb.refine_zlen - 1) / mb.refine_zlen);
         for (; i + 1 < n_normal; i += 2) {

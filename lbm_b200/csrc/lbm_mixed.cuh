@@ -29,7 +29,7 @@ struct MixedBuffers {
     float* rr = nullptr;
     int fuse_zlen = 0;           // >0: plain sweeps run two per pass, z runs of this length
     bool fuse_tall = false;      // ... on 32 x 16 tiles instead of 32 x 8
-    int refine_zlen = 0;         // z runs of the correction sweeps' passes (with fuse_zlen)
+    int refine_zlen = 0;         // the same for the refinement form's correction sweeps (tall tile)
     int collide_zlen = 0;        // >0: z-marching collide, z runs of this length
     bool allocated = false;
 };

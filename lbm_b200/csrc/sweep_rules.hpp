@@ -73,7 +73,7 @@ inline int fp64_pass_zlen(int lx, int ly, int lz, int sms)
 
 // Mixed: z run length of the passes (partial tiles store nothing outside the
 // box) and whether they take the tall tile; zlen 0 where single sweeps are
-// faster (zlen_tall: the tall tile's in any case).  Both sides' times on B200
+// faster.  Both sides' times on B200
 // (us per sweep): a pass takes 0.93 per wave and plane of its CTAs on 32 x 8
 // tiles (two per SM; 128^3: 29.8 at 34, 256^3: 226 at 238, 141 x 99 x 141: 31.9
 // at 36) and 0.91 on 32 x 16 (one per SM; 29.1, 223, 34.2 at 38).  A single
@@ -81,10 +81,21 @@ inline int fp64_pass_zlen(int lx, int ly, int lz, int sms)
 // cell; 80^3: 8.4, 64^3: 4.6, 32^3: 2.1), beyond 5.4 * 10^5 cells 20.5 per 10^6
 // cells less a remainder that stays there (84^3: 11.0, 88^3: 13.0, where the pass
 // takes 11.8), and 20.5 from DRAM (128^3: 45, 96^3: 18.4, 141 x 99 x 75: 27).
+//
+// The refinement form's correction sweeps read a source r of 15 values per cell
+// beside the 15 populations and take the tall tile: refine_zlen by a rule of
+// their own.  A pass takes 1.1 per wave and plane and 8 per 10^6 cells (128^3: 56.2
+// at 34, 136^3: 74.8 at 50, 136 x 98 x 177: 75.0 at 50, 88^3: 20.0 at 13); a single
+// sweep from DRAM, per 10^6 cells, 31 where rows are of whole 16 bytes (62.0, 76.6,
+// 71.2, 20.9), else 33 (91 x 98 x 73: 20.8, the pass 19.8), and 34 on tiles 16 cells
+// wide (45 x 183 x 190: 56.2, the pass 50.9).  With both sides measured on 144 boxes
+// of 5.4 * 10^5 to 1.7 * 10^7 cells this takes a form at most 3.6 % slower than the
+// other; the plain sweeps' rule took one up to 14 % slower (5 % where it chose
+// passes: 136 x 98 x 177).  Smaller boxes' single sweeps run from L2 (80^3: 14.2).
 struct MixedPass {
     int zlen = 0;
     bool tall = false;
-    int zlen_tall = 0;
+    int refine_zlen = 0;
 };
 inline MixedPass mixed_pass(int lx, int ly, int lz, int sms)
 {
@@ -93,15 +104,18 @@ inline MixedPass mixed_pass(int lx, int ly, int lz, int sms)
     if (!mixed_pass_fits(ly, n)) return m;
     long long low_cost = 0, tall_cost = 0;
     const int low = two_sweep_zlen(pass_tiles(lx, ly, S2_TX, S2_TY), lz, static_cast<long long>(S2_CTAS) * sms, &low_cost);
-    m.zlen_tall = two_sweep_zlen(pass_tiles(lx, ly, S2_TX, S2_TALL), lz, static_cast<long long>(S2_TALL_CTAS) * sms,
-                                 &tall_cost);
+    const int high = two_sweep_zlen(pass_tiles(lx, ly, S2_TX, S2_TALL), lz, static_cast<long long>(S2_TALL_CTAS) * sms,
+                                    &tall_cost);
     m.tall = tall_cost <= low_cost;
     const double mcells = 1e-6 * static_cast<double>(n);
     const double single = mcells <= 0.54   ? 1.75 + 13.0 * mcells
                           : mcells <= 0.75 ? 20.5 * mcells - 1.2
                                            : 20.5 * mcells;
     const double pass = m.tall ? 0.91 * static_cast<double>(tall_cost) : 0.93 * static_cast<double>(low_cost);
-    if (pass < single) m.zlen = m.tall ? m.zlen_tall : low;
+    if (pass < single) m.zlen = m.tall ? high : low;
+    const bool narrow = lx % 32 != 0 && lx <= 48;
+    const double correction = (narrow ? 34.0 : lx % 4 == 0 ? 31.0 : 33.0) * mcells;
+    if (mcells > 0.54 && 1.1 * static_cast<double>(tall_cost) + 8.0 * mcells < correction) m.refine_zlen = high;
     return m;
 }
 

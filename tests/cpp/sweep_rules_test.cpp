@@ -14,6 +14,11 @@ bool launchable(int lx, int ly, int lz, int tx, int ty, int zlen)
     return zlen >= 1 && zlen <= lz && gx <= 0x7fffffffLL && gy <= 65535 && gz <= 65535;
 }
 
+struct Box {
+    int lx, ly, lz;
+    bool passes;
+};
+
 }  // namespace
 
 int main()
@@ -25,6 +30,12 @@ int main()
     if (!fp64_pass_fits(6 * 65535, 6 * 65535) || fp64_pass_fits(6 * 65535 + 1, 6 * 65535 + 1)) return 2;
     if (!mixed_pass_fits(8 * 65535, 8 * 65535) || mixed_pass_fits(8 * 65535 + 1, 8 * 65535 + 1)) return 3;
     if (fp64_pass_fits(1, 143165577) || !fp64_pass_fits(1, 143165576)) return 4;
+    // correction sweeps of the refinement form: passes where they were measured 3 % or
+    // more faster, single sweeps where those were, whatever the plain sweeps take
+    for (const auto& b : {Box{88, 88, 88, true}, Box{128, 47, 100, true}, Box{96, 96, 96, true}, Box{118, 143, 129, true},
+                          Box{191, 141, 69, true}, Box{160, 160, 160, true}, Box{45, 183, 190, true}, Box{110, 57, 131, true}, Box{25, 161, 182, true}, Box{136, 98, 177, false}, Box{156, 88, 48, false},
+                          Box{64, 64, 64, false}, Box{130, 34, 150, false}, Box{33, 150, 150, false}})
+        if ((mixed_pass(b.lx, b.ly, b.lz, 148).refine_zlen > 0) != b.passes) return 9;
     const int extents[] = {1, 2, 3, 5, 6, 7, 8, 9, 16, 30, 31, 32, 33, 47, 64, 75, 96, 131, 203, 256, 1000, 65535, 393210, 393211,
                            524280, 524281, 4000000};
     long long chosen = 0;
@@ -38,7 +49,7 @@ int main()
                     if (z64 && !launchable(lx, ly, lz, F2_TX, F2_TY, z64)) return 5;
                     const MixedPass m = mixed_pass(lx, ly, lz, sms);
                     if (m.zlen && !launchable(lx, ly, lz, S2_TX, m.tall ? S2_TALL : S2_TY, m.zlen)) return 6;
-                    if (m.zlen && !launchable(lx, ly, lz, S2_TX, S2_TALL, m.zlen_tall)) return 7;
+                    if (m.refine_zlen && !launchable(lx, ly, lz, S2_TX, S2_TALL, m.refine_zlen)) return 7;
                     chosen += (z64 > 0) + (m.zlen > 0);
                 }
             }
