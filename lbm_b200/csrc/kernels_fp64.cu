@@ -1116,7 +1116,7 @@ void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double*
 void sweep_check_a(cudaStream_t st, const Launch& L, const Geom& g, const double* hin,
                    double* hout, double* p_chk, double* part)
 {
-    const bool planes = L.cnblocks < kCheckPlaneRuns;
+    const bool planes = L.check_planes();
     auto kern = planes ? sweep_check_a_kernel<kCheckZrun> : sweep_check_a_kernel<1>;
     kern<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, hin, hout, p_chk, part, L.cnblocks);
 }
@@ -1126,7 +1126,7 @@ void sweep_check_b(cudaStream_t st, const Launch& L, const Geom& g, bool dual, c
                    const double* s, const DevState* ds, double* part)
 {
     // (five terms of eight planes are more than a CTA's static shared memory)
-    const bool planes = !dual && L.cnblocks < kCheckPlaneRuns;
+    const bool planes = !dual && L.check_planes();
     auto kern = dual     ? sweep_check_b_kernel<true, 1>
                 : planes ? sweep_check_b_kernel<false, kCheckZrun>
                          : sweep_check_b_kernel<false, 1>;

@@ -663,7 +663,7 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
             sweep_kernel64<<<L.grid, L.block, 0, st>>>(g, mb.h[cur], mb.h[1 - cur], omega, mb.s);
         cur = 1 - cur;
     }
-    bool planes = L.cnblocks < kCheckPlaneRuns;
+    bool planes = L.check_planes();
     auto check_a = planes ? sweep_check_a_kernel<kCheckZrun> : sweep_check_a_kernel<1>;
     check_a<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.p_chk, mb.part_a, L.cnblocks);
     cur = 1 - cur;
@@ -745,7 +745,7 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
         cur = 1 - cur;
     }
     // the check sweep in FP64 on H + e
-    const bool planes = L.cnblocks < kRefinePlaneRuns;
+    const bool planes = L.refine_planes();
     auto check_a = planes ? refine_check_a_kernel<kCheckZrun> : refine_check_a_kernel<1>;
     check_a<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, H, e, Hn, mb.p_chk, mb.part_a, L.cnblocks);
     finalize(st, FIN_SIGMA, ds, mb.part_a, L.cnblocks, nullptr, 0, nullptr, 0);

@@ -1183,6 +1183,7 @@ lbm_status lbm_create(const lbm_params* prm, lbm_precision precision, int device
     h->phys = make_phys(*prm);
     const int bx = pick_bx(prm->lx);
     h->L = make_launch(prm->lx, prm->ly, prm->lz, bx, 256 / bx);
+    set_check_planes(h->L, prop.multiProcessorCount);
     lbm_status st = LBM_OK;
     auto bail = [&](lbm_status s) {
         free_all(h);

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <cstdlib>
 
 #include "../../include/lbm_b200.h"
 #include "lbm_device.cuh"
@@ -79,22 +80,32 @@ struct Launch {
     dim3 cgrid;
     long long cnblocks;
     int zrun;
+    // Runs below which checks A and B go a plane per CTA (set_check_planes), and the
+    // refinement form's.
+    long long plane_runs = 0, refine_plane_runs = 0;
+    bool check_planes() const { return cnblocks < plane_runs && cgrid.z <= kMaxGridY / kCheckZrun; }
+    bool refine_planes() const { return cnblocks < refine_plane_runs && cgrid.z <= kMaxGridY / kCheckZrun; }
     // Grid of a check kernel that runs a plane per CTA, clusters of kCheckZrun
     // making a run (zrun_terms); else cgrid.
     dim3 check_grid(bool planes) const { return planes ? dim3(cgrid.x, cgrid.y, cgrid.z * kCheckZrun) : cgrid; }
 };
 
-// Runs below which checks A and B go a plane per CTA: with one CTA per run a
-// check of a small box is eight planes one after another on a few SMs (32^3: 16
-// CTAs).  Per sweep of a check interval of 100, us, a run per CTA and a plane per
+// With one CTA per run a check of a small box is eight planes one after another on
+// a few SMs (32^3: 16 CTAs), so it goes a plane per CTA while there are fewer runs
+// than SMs.  Per sweep of a check interval of 100, us, a run per CTA and a plane per
 // CTA: FP64 2.81 and 2.69 at 32^3 (16 runs), 4.26 and 4.20 at 48^3 (72), 7.84
 // both at 64^3 (128), 14.39 and 14.43 at 72^3 (243); FP32 2.08 and 1.95, 2.95 and
-// 2.79, 4.88 and 4.82, 7.10 both, 12.91 and 13.10 at 88^3 (363).
-constexpr long long kCheckPlaneRuns = 148;
-// The refinement form's, in FP64 on H + e: 2.49 and 2.19 at 32^3, 6.18 and 5.90
-// at 64^3, 14.45 and 14.14 at 80^3 (300), 37.1 and 36.9 at 104^3 (676), 59.3 and
-// 59.4 at 128^3 (1024).
-constexpr long long kRefinePlaneRuns = 740;
+// 2.79, 4.88 and 4.82, 7.10 both, 12.91 and 13.10 at 88^3 (363).  The refinement
+// form's, in FP64 on H + e, below five runs per SM: 2.49 and 2.19 at 32^3, 6.18 and
+// 5.90 at 64^3, 14.45 and 14.14 at 80^3 (300), 37.1 and 36.9 at 104^3 (676), 59.3 and
+// 59.4 at 128^3 (1024).  LBM_CHECK_PLANES: 0 never, 1 always.
+inline void set_check_planes(Launch& L, int sms)
+{
+    const char* env = std::getenv("LBM_CHECK_PLANES");
+    const long long always = 1LL << 62;
+    L.plane_runs = !env ? sms : (env[0] == '0' ? 0 : always);
+    L.refine_plane_runs = !env ? 5LL * sms : L.plane_runs;
+}
 
 inline Launch make_launch(int lx, int ly, int lz, int bx, int by)
 {
