@@ -18,6 +18,7 @@
 #include <math_constants.h>
 
 #include <cstdlib>
+#include <cstring>
 
 #include "collide_zm.cuh"
 #include "lbm_mixed.cuh"
@@ -506,7 +507,10 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
     mb.refine_zlen = 0;
     int zlen = 0, refine_zlen = 0;
     if (const char* env = std::getenv("LBM_SWEEP2_ZLEN")) {
+        // n: z runs of n planes on 32 x 8 tiles; nx16: on 32 x 16
         zlen = refine_zlen = std::atoi(env);
+        const char* x = std::strchr(env, 'x');
+        mb.fuse_tall = x && std::atoi(x + 1) == S2_TALL;
     } else {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess ||
