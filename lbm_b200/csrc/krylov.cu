@@ -275,16 +275,18 @@ namespace {
 // (which takes the inner products) run in pairs: the rule and the z runs of the
 // FP64 box's two-sweep passes, 0 elsewhere.  At 128^3 a pair takes 120 us, two
 // single applications 170 to 190; a degree-8 iteration 1.81 instead of 2.16 ms.
-// LBM_KRYLOV_PAIRS=0 turns them off.
+// LBM_KRYLOV_PAIRS=0 turns them off, =zN runs them on z runs of N planes wherever
+// they fit.
 int pair_run(const Geom& g)
 {
     const char* env = std::getenv("LBM_KRYLOV_PAIRS");
     if (env && env[0] == '0') return 0;
+    const int forced = env && env[0] == 'z' && fp64_pass_fits(g.ly, g.n) ? std::atoi(env + 1) : 0;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
-    const int zlen = fp64_pass_zlen(g.lx, g.ly, g.lz, sms);
+    const int zlen = forced > 0 ? forced : fp64_pass_zlen(g.lx, g.ly, g.lz, sms);
     return zlen > 0 && cudaFuncSetAttribute(apply2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             f2_smem(ApplyOps::kCoefs)) == cudaSuccess
                ? zlen
@@ -335,6 +337,7 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
             double* dst = src == kb.w1 ? kb.w2 : kb.w1;
             if (j > 1 && j + 1 < m && pair_zlen > 0) {
                 apply2_kernel<<<f2_grid(g, pair_zlen), F2_RC, f2_smem(ApplyOps::kCoefs), st>>>(g, pair_zlen, src, dst, rho);
+                ++res->pairs;
                 j += 2;
             } else {
                 const bool sum_p = border && j == 1;
@@ -350,10 +353,13 @@ lbm_status bicgstab(cudaStream_t st, const Launch& L, const Geom& g, const Krylo
     };
     // y = the update and A y into kb.w1, returning 1; 0 where the update is a
     // launch of its own: degree 1, whose one application reads y at its own
-    // cells too, and the adjoint, whose walls read some elements twice
+    // cells too, the adjoint, whose walls read some elements twice, and
+    // LBM_KRYLOV_UPDATES=0
+    const char* uenv = std::getenv("LBM_KRYLOV_UPDATES");
+    const bool own_updates = kAdj || m == 1 || (uenv && uenv[0] == '0');
     auto update_apply = [&](auto opc, double a0, double a1, double* y, const double* x0, const double* x1) -> int {
         constexpr int kOp = decltype(opc)::value;
-        if (kAdj || m == 1) {
+        if (own_updates) {
             vec_kernel<kOp><<<kDotBlocks, 256, 0, st>>>(cnt, a0, a1, y, nullptr, x0, x1, nullptr, nullptr, nullptr);
             return 0;
         }

@@ -780,6 +780,7 @@ lbm_status step_once(lbm_handle* h, uint64_t replay, lbm_step_stats* stats)
             return fail(h, LBM_ERR_POISSON_BUDGET, "Poisson sweep limit reached without convergence");
         iters = kr.matvecs;
         kernels = kr.matvecs;
+        fused_sweeps = 2 * kr.pairs;
         launches += 4 * kr.iterations + 6;
         dh.iterations = kr.matvecs;
         dh.rel = kr.rel_residual;

@@ -249,6 +249,7 @@ struct KrylovBuffers {
 struct KrylovResult {
     uint64_t matvecs = 0;      // applications of (I - K): two per iteration plus the initial residual
     uint64_t iterations = 0;
+    uint64_t pairs = 0;        // launches that applied K twice
     uint64_t restarts = 0;     // restarts from the true residual (near-breakdown, every 200 iterations)
     double rel_residual = 0.0; // ||b - (I - K) h|| / ||b|| at exit (the recurrence's)
     double gauge_shift = 0.0;
