@@ -440,6 +440,12 @@ int lbm_abi_version(void);
  * numerator infinite); *mismatches = pairs whose bits differ. */
 lbm_status lbm_selftest_division(uint64_t samples, uint64_t seed, uint64_t* mismatches);
 
+/* Self-check of the adjoint's transposed pull on a box of at most 2^24 cells: the
+ * form that loads all populations of a cell before the slip walls' transposed
+ * overwrite against that of one population at a time; *mismatches = values whose
+ * bits differ. */
+lbm_status lbm_selftest_transposed_pull(int lx, int ly, int lz, int periodic_x, uint64_t* mismatches);
+
 /* ---- batched boxes ------------------------------------------------------
  * Many independent droplet boxes of different sizes and physics advanced
  * together on one GPU, mixed precision (FP32 populations, FP64 pressure sums,

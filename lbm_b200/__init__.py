@@ -196,6 +196,7 @@ def load_library(path: str = LIB_PATH):
     L.lbm_status_string.restype = C.c_char_p
     L.lbm_abi_version.restype = C.c_int
     L.lbm_selftest_division.argtypes = [C.c_uint64, C.c_uint64, C.POINTER(C.c_uint64)]
+    L.lbm_selftest_transposed_pull.argtypes = [C.c_int] * 4 + [C.POINTER(C.c_uint64)]
     B = C.c_void_p
     L.lbm_batch_create.argtypes = [C.POINTER(Params), C.c_int, C.c_int, C.POINTER(B)]
     L.lbm_batch_destroy.argtypes = [B]
@@ -675,6 +676,16 @@ def selftest_division(samples: int = 1 << 30, seed: int = 12345) -> int:
     st = lib.lbm_selftest_division(samples, seed, C.byref(out))
     if st != 0:
         raise LBMError(st, "lbm_selftest_division")
+    return int(out.value)
+
+
+def selftest_transposed_pull(lx: int, ly: int, lz: int, periodic_x: bool) -> int:
+    """lbm_selftest_transposed_pull: values of the adjoint's transposed pull for
+    which its two forms differ."""
+    out = C.c_uint64(0)
+    st = load_library().lbm_selftest_transposed_pull(lx, ly, lz, int(periodic_x), C.byref(out))
+    if st != 0:
+        raise LBMError(st, "lbm_selftest_transposed_pull")
     return int(out.value)
 
 

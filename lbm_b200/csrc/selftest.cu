@@ -1,11 +1,15 @@
 // selftest.cu -- lbm_selftest_division: the FP64 kernels' division from
 // a reciprocal pair (exact_div.cuh) against CUDA's IEEE division on
 // pseudo-random operands of the kinds the kernels use, infinite numerators
-// among them.
+// among them.  lbm_selftest_transposed_pull: the transposed pull of all
+// populations at once (tpull_all) against that of one at a time (tpull).
 #include <cuda_runtime.h>
+
+#include <vector>
 
 #include "../../include/lbm_b200.h"
 #include "exact_div.cuh"
+#include "lbm_device.cuh"
 
 namespace {
 
@@ -55,7 +59,58 @@ __global__ void division_selftest_kernel(unsigned long long n, unsigned long lon
     if (bad) atomicAdd(mismatches, bad);
 }
 
+template <class I>
+__global__ void transposed_pull_kernel(lbm::Geom g, const double* __restrict__ y, unsigned long long* __restrict__ mismatches)
+{
+    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (c >= g.n) return;
+    const int x = static_cast<int>(c % g.lx), yy = static_cast<int>(c / g.lx % g.ly), z = static_cast<int>(c / g.lx / g.ly);
+    const I n = static_cast<I>(g.n);
+    const lbm::Wrap w(g, x, yy, z);
+    double m[lbm::Q];
+    lbm::tpull_all(m, y, n, g, w, x, yy, z);
+    int bad = 0;
+    lbm::static_for<0, lbm::Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        bad += __double_as_longlong(m[q]) != __double_as_longlong(lbm::tpull<q>(y, n, g, w, x, yy, z));
+    });
+    if (bad) atomicAdd(mismatches, static_cast<unsigned long long>(bad));
+}
+
 }  // namespace
+
+extern "C" lbm_status lbm_selftest_transposed_pull(int lx, int ly, int lz, int periodic_x, uint64_t* mismatches)
+{
+    if (!mismatches || lx < 2 || ly < 1 || lz < 1 || static_cast<long long>(lx) * ly * lz > (1 << 24)) return LBM_ERR_BAD_ARG;
+    lbm::Geom g{};
+    g.lx = lx;
+    g.ly = ly;
+    g.lz = lz;
+    g.periodic_x = periodic_x ? 1 : 0;
+    g.n = static_cast<long long>(lx) * ly * lz;
+    const size_t count = lbm::Q * static_cast<size_t>(g.n);
+    std::vector<double> host(count);
+    for (size_t i = 0; i < count; ++i) host[i] = static_cast<double>(i + 1) / 7.0;
+    double* y = nullptr;
+    unsigned long long* d = nullptr;
+    if (cudaMalloc(&y, count * sizeof(double)) != cudaSuccess || cudaMalloc(&d, sizeof(*d)) != cudaSuccess) {
+        cudaFree(y);
+        cudaGetLastError();
+        return LBM_ERR_OOM;
+    }
+    cudaMemcpy(y, host.data(), count * sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemset(d, 0, sizeof(*d));
+    const unsigned blocks = static_cast<unsigned>((g.n + 255) / 256);
+    transposed_pull_kernel<int><<<blocks, 256>>>(g, y, d);
+    transposed_pull_kernel<long long><<<blocks, 256>>>(g, y, d);
+    unsigned long long h = 0;
+    const bool ok = cudaGetLastError() == cudaSuccess && cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess;
+    cudaFree(y);
+    cudaFree(d);
+    if (!ok) return LBM_ERR_CUDA;
+    *mismatches = h;
+    return LBM_OK;
+}
 
 extern "C" lbm_status lbm_selftest_division(uint64_t samples, uint64_t seed, uint64_t* mismatches)
 {
