@@ -1124,14 +1124,39 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
     const int ctas[3] = {2, 4, 8};
     lbm_batch_tuning best = b->tune;
     best.sweep_ms = 1e30;
-    // A form's time per launch, in a graph as the segments are (launched one by one
-    // the sweeps of small boxes wait for the host, single sweeps the longest).
     const int reps = 6;
-    auto time_launches = [&](int launches, auto&& launch, double* ms_each) -> lbm_status {
+    auto singles = [&](const lbm_batch_tuning& t, int first, int count) {
+        for (int r = first; r < first + count; ++r)
+            b_sweep<<<grid_of(b), 256, 0, st>>>(b->items_d, b->n_items, b->inst_d, t.tile_x, b->ctl, r, b->pool);
+    };
+    for (auto& tl : tiles)
+        for (int zr : zruns)
+            for (int cp : ctas) {
+                const lbm_batch_tuning t{tl[0], tl[1], zr, cp, 0, 0, 0.0};
+                b->tune = t;
+                lbm_status s = build_items(b);
+                if (s != LBM_OK) return s;
+                singles(t, 0, 2);
+                BCUDA(b, cudaEventRecord(b->ev[0], st));
+                singles(t, 0, reps);
+                BCUDA(b, cudaEventRecord(b->ev[1], st));
+                BCUDA(b, cudaGetLastError());
+                BCUDA(b, cudaEventSynchronize(b->ev[1]));
+                float ms = 0.f;
+                cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
+                if (ms / reps < best.sweep_ms) {
+                    best = t;
+                    best.sweep_ms = ms / reps;
+                }
+            }
+    // Single sweeps against passes: each in a graph, as the segments run them
+    // (launched one by one the sweeps of small boxes wait for the host, single
+    // sweeps the longest).  *ms: time per sweep of `sweeps` sweeps.
+    auto time_graph = [&](int sweeps, auto&& launch, double* ms) -> lbm_status {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t ex = nullptr;
         cudaError_t e = capture_graph(st, &graph, [&] {
-            for (int r = 0; r < launches; ++r) launch(r);
+            launch();
             return cudaSuccess;
         });
         BCUDA(b, e);
@@ -1143,32 +1168,20 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
         if (e == cudaSuccess) e = cudaGraphLaunch(ex, st);
         if (e == cudaSuccess) e = cudaEventRecord(b->ev[1], st);
         if (e == cudaSuccess) e = cudaEventSynchronize(b->ev[1]);
-        float ms = 0.f;
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
+        float t = 0.f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&t, b->ev[0], b->ev[1]);
         cudaGraphExecDestroy(ex);
         BCUDA(b, e);
-        *ms_each = ms / launches;
+        *ms = t / sweeps;
         return LBM_OK;
     };
-    for (auto& tl : tiles)
-        for (int zr : zruns)
-            for (int cp : ctas) {
-                const lbm_batch_tuning t{tl[0], tl[1], zr, cp, 0, 0, 0.0};
-                b->tune = t;
-                lbm_status s = build_items(b);
-                if (s != LBM_OK) return s;
-                const int grid = grid_of(b);
-                double ms = 0.0;
-                s = time_launches(reps, [&](int r) {
-                    b_sweep<<<grid, 256, 0, st>>>(b->items_d, b->n_items, b->inst_d, t.tile_x, b->ctl, r, b->pool);
-                }, &ms);
-                if (s != LBM_OK) return s;
-                if (ms < best.sweep_ms) {
-                    best = t;
-                    best.sweep_ms = ms;
-                }
-            }
+    b->tune = best;
+    lbm_status ts = build_items(b);
+    if (ts == LBM_OK) ts = time_graph(reps, [&] { singles(best, 0, reps); }, &best.sweep_ms);
+    if (ts != LBM_OK) return ts;
     // two sweeps per launch on z runs of 8, 16, 32 (per-sweep time = launch / 2)
+    // where that is worth the plan that a segment of passes starts with (some 3 us)
+    double least = 0.98 * best.sweep_ms;
     const int zr2[3] = {8, 16, 32};
     for (int zr : zr2) {
         lbm_batch_tuning t = best;
@@ -1179,11 +1192,13 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
         if (s != LBM_OK) return s;
         enqueue_plan2(b, st);
         double ms = 0.0;
-        s = time_launches(reps / 2, [&](int r) { enqueue_sweep2(b, r, st); }, &ms);
+        s = time_graph(reps, [&] {
+            for (int r = 0; r < reps / 2; ++r) enqueue_sweep2(b, r, st);
+        }, &ms);
         if (s != LBM_OK) return s;
-        if (ms / 2.0 < best.sweep_ms) {
+        if (ms < least) {
             best = t;
-            best.sweep_ms = ms / 2.0;
+            best.sweep_ms = least = ms;
         }
     }
     b->tune = best;
