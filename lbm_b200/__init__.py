@@ -260,10 +260,8 @@ def _page_allocator():
         from numpy.core import _multiarray_umath as core
     if not hasattr(core, "get_handler_name"):
         return None
-    pointer = C.pythonapi.PyCapsule_GetPointer
-    pointer.restype, pointer.argtypes = C.c_void_p, [C.py_object, C.c_char_p]
-    capsule = C.pythonapi.PyCapsule_New
-    capsule.restype, capsule.argtypes = C.py_object, [C.c_void_p, C.c_char_p, C.c_void_p]
+    pointer = C.PYFUNCTYPE(C.c_void_p, C.py_object, C.c_char_p)(("PyCapsule_GetPointer", C.pythonapi))
+    capsule = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_char_p, C.c_void_p)(("PyCapsule_New", C.pythonapi))
     api = C.cast(pointer(core._ARRAY_API, None), C.POINTER(C.c_void_p))
     set_handler = C.PYFUNCTYPE(C.py_object, C.py_object)(api[304])   # its slot in NumPy's C API since 1.22
     table = load_library().lbm_host_pages
