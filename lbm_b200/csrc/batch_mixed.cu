@@ -729,18 +729,23 @@ bool get_loop(lbm_batch* b, int n_normal, cudaGraphExec_t* out)
     if (!b->loop_segs) {
         if (cudaMalloc(&b->loop_segs, sizeof(unsigned)) != cudaSuccess) {
             b->loop_segs = nullptr;
+            cudaGetLastError();   // (the host loop takes over: no error of its captures)
             return false;
         }
         if (cudaMallocHost(&b->loop_segs_host, sizeof(unsigned)) != cudaSuccess) {
             cudaFree(b->loop_segs);
             b->loop_segs = nullptr;
             b->loop_segs_host = nullptr;
+            cudaGetLastError();
             return false;
         }
     }
     cudaStream_t st = b->stream;
     cudaGraph_t top = nullptr;
-    if (cudaGraphCreate(&top, 0) != cudaSuccess) return false;
+    if (cudaGraphCreate(&top, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     cudaGraphExec_t ex = nullptr;
     cudaError_t e = cudaSuccess;
     cudaGraphConditionalHandle hw = 0;

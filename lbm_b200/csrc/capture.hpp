@@ -15,8 +15,8 @@ namespace lbm {
 
 // Captures what enqueue() -> cudaError_t launches on st; *graph is the caller's
 // to destroy on cudaSuccess, null otherwise.  Returns the first error of the
-// capture's start, enqueue, its launches and the capture's end; st does not
-// capture afterwards.
+// capture's start, enqueue, its launches (or one not looked at before them) and
+// the capture's end; st does not capture afterwards.
 template <class F>
 cudaError_t capture_graph(cudaStream_t st, cudaGraph_t* graph, F&& enqueue)
 {

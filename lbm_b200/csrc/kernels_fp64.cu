@@ -1102,9 +1102,7 @@ void sweep(cudaStream_t st, const Launch& L, const Geom& g, const double* hin, d
 
 bool sweep2_prepare(const Geom& g)
 {
-    return fp64_pass_fits(g.ly, g.n) &&
-           cudaFuncSetAttribute(sweep2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                f2_smem(SweepOps::kCoefs)) == cudaSuccess;
+    return fp64_pass_fits(g.ly, g.n) && allow_smem(sweep2_kernel, f2_smem(SweepOps::kCoefs));
 }
 
 void sweep2(cudaStream_t st, const Geom& g, int zlen, const double* hin, double* hout,

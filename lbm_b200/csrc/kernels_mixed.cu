@@ -522,10 +522,8 @@ lbm_status mixed_alloc(MixedBuffers& mb, const Geom& g, const Launch& L)
         mb.fuse_tall = m.tall;
     }
     if ((zlen > 0 || refine_zlen > 0) && mixed_pass_fits(g.ly, g.n) &&
-        cudaFuncSetAttribute(sweep2_kernel<S2_TALL, S2_TALL_CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess &&
-        cudaFuncSetAttribute(sweep2_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             sweep2_smem(S2_TX, S2_TALL)) == cudaSuccess) {
+        allow_smem(sweep2_kernel<S2_TALL, S2_TALL_CTAS>, sweep2_smem(S2_TX, S2_TALL)) &&
+        allow_smem(sweep2_refine_kernel, sweep2_smem(S2_TX, S2_TALL))) {
         mb.fuse_zlen = zlen > 0 ? zlen : 0;
         mb.refine_zlen = refine_zlen > 0 ? refine_zlen : 0;
     }

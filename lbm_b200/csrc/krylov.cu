@@ -287,10 +287,7 @@ int pair_run(const Geom& g)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
     const int zlen = forced > 0 ? forced : fp64_pass_zlen(g.lx, g.ly, g.lz, sms);
-    return zlen > 0 && cudaFuncSetAttribute(apply2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            f2_smem(ApplyOps::kCoefs)) == cudaSuccess
-               ? zlen
-               : 0;
+    return zlen > 0 && allow_smem(apply2_kernel, f2_smem(ApplyOps::kCoefs)) ? zlen : 0;
 }
 
 // BiCGSTAB iterations on (I - A_op) h = b from the initial guess in h; the

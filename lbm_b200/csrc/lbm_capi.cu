@@ -480,12 +480,14 @@ bool get_loop(lbm_handle* h, const SegKey& key, cudaGraphExec_t* out, int* end_p
     if (!h->loopctl) {
         if (cudaMalloc(&h->loopctl, sizeof(LoopCtl)) != cudaSuccess) {
             h->loopctl = nullptr;
+            cudaGetLastError();   // (the host loop takes over: no error of its captures)
             return false;
         }
         if (cudaMallocHost(&h->loopctl_host, sizeof(LoopCtl)) != cudaSuccess) {
             cudaFree(h->loopctl);
             h->loopctl = nullptr;
             h->loopctl_host = nullptr;
+            cudaGetLastError();
             return false;
         }
     }

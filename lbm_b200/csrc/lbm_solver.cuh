@@ -141,6 +141,16 @@ inline SweepShape sweep_shape(const Launch& L, const Geom& g, int threads)
 constexpr int kSweepThreads64 = 32;
 inline int sweep_threads32(const Geom& g) { return g.n < (1 << 16) ? 128 : 64; }
 
+// Lets a kernel have `bytes` of dynamic shared memory; where it may not, the caller
+// takes another form, so no error is left behind.
+template <class Kernel>
+bool allow_smem(Kernel kernel, int bytes)
+{
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Buffers of one FP64 box.  Populations are q-major SoA: a[q*n + cell].
 struct Fp64Buffers {
     double* f[2];       // post-collision f* ping-pong

@@ -75,6 +75,10 @@ int main()
     if (lbm::capture_graph(nullptr, &graph, refused) != cudaErrorInvalidConfiguration || graph || graphs || ended != 1 ||
         pending != cudaSuccess)
         return 3;
+    // a launch refused ahead of the capture, not looked at yet: reported as well
+    reset();
+    pending = cudaErrorInvalidValue;
+    if (lbm::capture_graph(nullptr, &graph, fine) != cudaErrorInvalidValue || graph || graphs || ended != 1) return 6;
     // a failing copy among the launches
     reset();
     const auto copy = [] { return cudaErrorInvalidValue; };
