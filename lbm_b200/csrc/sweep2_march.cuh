@@ -16,8 +16,8 @@
 // What bounds it: FP64 latency and the two barriers at 16 warps per SM; 126
 // registers (15 populations in flight and 15 at work) allow no more, and fewer
 // registers spill (0.54 ms per sweep at 96 registers, 0.62 at 80).  Measured on
-// B200 at 256^3, ms per sweep: 0.42 (5.1 TB/s of the 128 B/cell it moves)
-// against 0.65 for single sweeps; other shapes: 32 x 8 tiles with 11 warps in
+// B200 at 256^3, ms per sweep: 0.444 (4.8 TB/s of the 128 B/cell it moves)
+// against 0.657 for single sweeps; other shapes: 32 x 8 tiles with 11 warps in
 // one CTA 0.45, 30 x 14 in one CTA 0.47, 16 x 12 0.47; neighbouring warps
 // joined by named barriers in place of the CTA barriers 0.44; separate warps
 // for the two sweeps 0.47; the rows requested into L2 a plane ahead 0.48.
