@@ -412,7 +412,7 @@ poisson_init_kernel(Geom g, int h_loaded, const double* __restrict__ hload,
     const long long c = cell_of(g, x, y, z);
     const double pv = p[c];
     const double tauh = 1.0 / rho[c] + 0.5;
-    const RecipPair rt = recip_for(recip_pair(tauh), pv);
+    const RecipPair rt = recip_for_branch(recip_pair(tauh), pv);
     const double sv = s[c];
     static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
@@ -427,12 +427,12 @@ poisson_init_kernel(Geom g, int h_loaded, const double* __restrict__ hload,
 }
 
 // Kinetic collision of one population, h - (h - E p) / tau - (E / 3) s
-// (CPU/Inamuro.cpp:755-778), the quotient from tau's reciprocal pair.
+// (CPU/Inamuro.cpp:755-778), the quotient from tau's reciprocal pair (recip_for).
 template <int q>
 __device__ __forceinline__ double collide_h(double h, double pv, const RecipPair& rt, double sv)
 {
     constexpr double E = wE(q);
-    return h - div_rn(h - E * pv, recip_for(rt, pv)) - (E / 3.0) * sv;
+    return h - div_rn(h - E * pv, rt) - (E / 3.0) * sv;
 }
 
 // I: index type (long long in general, int where 15 n < 2^31).
@@ -440,7 +440,8 @@ template <class I>
 __device__ __forceinline__ void collide_h_store(const double (&hv)[Q], double pv, double tauh,
                                                 double sv, double* __restrict__ hout, I n, I c)
 {
-    const RecipPair rt = recip_pair(tauh);   // the 15 quotients by tau_h come from it (exact_div.cuh)
+    // the 15 quotients by tau_h come from it (exact_div.cuh)
+    const RecipPair rt = recip_for_branch(recip_pair(tauh), pv);
     static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
         hout[(I)q * n + c] = collide_h<q>(hv[q], pv, rt, sv);
@@ -500,7 +501,7 @@ struct SweepOps {
     template <int q>
     static __device__ __forceinline__ double collide(double h, double pv, const double (&k)[3])
     {
-        return collide_h<q>(h, pv, RecipPair{k[0], k[1]}, k[2]);
+        return collide_h<q>(h, pv, recip_for(RecipPair{k[0], k[1]}, pv), k[2]);
     }
 };
 

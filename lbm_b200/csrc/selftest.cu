@@ -53,8 +53,10 @@ __global__ void division_selftest_kernel(unsigned long long n, unsigned long lon
         default: b = random_double(r2, -200, 200, true); break;   // any normal divisor
         }
         const double q = lbm::div_rn(a, lbm::recip_for(lbm::recip_pair(b), p));
+        const double qb = lbm::div_rn(a, lbm::recip_for_branch(lbm::recip_pair(b), p));
         const double ref = __ddiv_rn(a, b);
-        if (__double_as_longlong(q) != __double_as_longlong(ref)) ++bad;
+        if (__double_as_longlong(q) != __double_as_longlong(ref) || __double_as_longlong(qb) != __double_as_longlong(ref))
+            ++bad;
     }
     if (bad) atomicAdd(mismatches, bad);
 }
