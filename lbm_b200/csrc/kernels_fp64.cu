@@ -514,7 +514,7 @@ sweep2_kernel(Geom g, int zlen, const double* __restrict__ hin, double* __restri
 }
 
 template <int kPlanes>
-__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 sweep_check_a_kernel(Geom g, int zrun, const double* __restrict__ hin, double* __restrict__ hout,
                      double* __restrict__ p_chk, double* __restrict__ part, long long nblocks)
 {
@@ -538,7 +538,7 @@ sweep_check_a_kernel(Geom g, int zrun, const double* __restrict__ hin, double* _
 }
 
 template <bool kDual, int kPlanes>
-__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 sweep_check_b_kernel(Geom g, int zrun, const double* __restrict__ hin, double* __restrict__ hout,
                      double* __restrict__ hc,
                      const double* __restrict__ p_chk, double* __restrict__ p_prev,
@@ -1117,7 +1117,7 @@ void sweep_check_a(cudaStream_t st, const Launch& L, const Geom& g, const double
 {
     const bool planes = L.check_planes();
     auto kern = planes ? sweep_check_a_kernel<kCheckZrun> : sweep_check_a_kernel<1>;
-    kern<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, hin, hout, p_chk, part, L.cnblocks);
+    launch_check(st, L, planes, kern, g, L.zrun, hin, hout, p_chk, part, L.cnblocks);
 }
 
 void sweep_check_b(cudaStream_t st, const Launch& L, const Geom& g, bool dual, const double* hin, double* hout,
@@ -1129,7 +1129,7 @@ void sweep_check_b(cudaStream_t st, const Launch& L, const Geom& g, bool dual, c
     auto kern = dual     ? sweep_check_b_kernel<true, 1>
                 : planes ? sweep_check_b_kernel<false, kCheckZrun>
                          : sweep_check_b_kernel<false, 1>;
-    kern<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, hin, hout, hc, p_chk, p_prev, p, rho, s, ds, part,
+    launch_check(st, L, planes, kern, g, L.zrun, hin, hout, hc, p_chk, p_prev, p, rho, s, ds, part,
                                                    L.cnblocks);
 }
 

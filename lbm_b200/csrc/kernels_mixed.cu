@@ -224,7 +224,7 @@ sweep2_refine_kernel(Geom g, int zlen, const float* __restrict__ ein, float* __r
 }
 
 template <int kPlanes>
-__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 sweep_check_a_kernel(Geom g, int zrun, const float* __restrict__ hin, float* __restrict__ hout,
                      double* __restrict__ p_chk, double* __restrict__ part, long long nblocks)
 {
@@ -237,7 +237,7 @@ sweep_check_a_kernel(Geom g, int zrun, const float* __restrict__ hin, float* __r
 }
 
 template <bool kDual, int kPlanes>
-__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 sweep_check_b_kernel(Geom g, int zrun, const float* __restrict__ hin, float* __restrict__ hout,
                      float* __restrict__ hc,
                      const double* __restrict__ p_chk, double* __restrict__ p_prev,
@@ -369,7 +369,7 @@ refine_sweep_kernel(Geom g, const float* __restrict__ ein, float* __restrict__ e
 // Check A in FP64: pull H + e, slip, p = sum (FP64); the uncollided values
 // go to hpre, red[0] += p.
 template <int kPlanes>
-__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 refine_check_a_kernel(Geom g, int zrun, const double* __restrict__ hd, const float* __restrict__ e,
                       double* __restrict__ hpre, double* __restrict__ p_chk, double* __restrict__ part,
                       long long nblocks)
@@ -402,7 +402,7 @@ refine_check_a_kernel(Geom g, int zrun, const double* __restrict__ hd, const flo
 // Check B in FP64: gauge (p -= shift, h -= E shift), relative-change terms,
 // p and p_prev, then the collision of the next sweep, in place.
 template <int kPlanes>
-__global__ void __cluster_dims__(1, 1, kPlanes) __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 refine_check_b_kernel(Geom g, int zrun, double* __restrict__ hd, const double* __restrict__ p_chk,
                       double* __restrict__ p_prev, double* __restrict__ p, const float* __restrict__ omega,
                       const float* __restrict__ s, const DevState* __restrict__ ds, double* __restrict__ part,
@@ -667,7 +667,7 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
     }
     bool planes = L.check_planes();
     auto check_a = planes ? sweep_check_a_kernel<kCheckZrun> : sweep_check_a_kernel<1>;
-    check_a<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.p_chk, mb.part_a, L.cnblocks);
+    launch_check(st, L, planes, check_a, g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.p_chk, mb.part_a, L.cnblocks);
     cur = 1 - cur;
     finalize(st, FIN_SIGMA, ds, mb.part_a, L.cnblocks, nullptr, 0, nullptr, 0);
     // (five terms of eight planes are more than a CTA's static shared memory)
@@ -675,7 +675,7 @@ int mixed_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, const Geom
     auto check_b = dual     ? sweep_check_b_kernel<true, 1>
                    : planes ? sweep_check_b_kernel<false, kCheckZrun>
                             : sweep_check_b_kernel<false, 1>;
-    check_b<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.hc, mb.p_chk, mb.p_prev,
+    launch_check(st, L, planes, check_b, g, L.zrun, mb.h[cur], mb.h[1 - cur], mb.hc, mb.p_chk, mb.p_prev,
                                                       mb.p, omega, mb.s, ds, mb.part_b, L.cnblocks);
     cur = 1 - cur;
     if (dual) {
@@ -749,10 +749,10 @@ int mixed_refine_segment(cudaStream_t st, MixedBuffers& mb, const Launch& L, con
     // the check sweep in FP64 on H + e
     const bool planes = L.refine_planes();
     auto check_a = planes ? refine_check_a_kernel<kCheckZrun> : refine_check_a_kernel<1>;
-    check_a<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, H, e, Hn, mb.p_chk, mb.part_a, L.cnblocks);
+    launch_check(st, L, planes, check_a, g, L.zrun, H, e, Hn, mb.p_chk, mb.part_a, L.cnblocks);
     finalize(st, FIN_SIGMA, ds, mb.part_a, L.cnblocks, nullptr, 0, nullptr, 0);
     auto check_b = planes ? refine_check_b_kernel<kCheckZrun> : refine_check_b_kernel<1>;
-    check_b<<<L.check_grid(planes), L.block, 0, st>>>(g, L.zrun, Hn, mb.p_chk, mb.p_prev, mb.p, omega, mb.s, ds,
+    launch_check(st, L, planes, check_b, g, L.zrun, Hn, mb.p_chk, mb.p_prev, mb.p, omega, mb.s, ds,
                                                       mb.part_b, L.cnblocks);
     finalize(st, FIN_CHECK, ds, mb.part_b, L.cnblocks, nullptr, 0, nullptr, 0);
     return 1 - start_parity;

@@ -85,9 +85,6 @@ struct Launch {
     long long plane_runs = 0, refine_plane_runs = 0;
     bool check_planes() const { return cnblocks < plane_runs && cgrid.z <= kMaxGridY / kCheckZrun; }
     bool refine_planes() const { return cnblocks < refine_plane_runs && cgrid.z <= kMaxGridY / kCheckZrun; }
-    // Grid of a check kernel that runs a plane per CTA, clusters of kCheckZrun
-    // making a run (zrun_terms); else cgrid.
-    dim3 check_grid(bool planes) const { return planes ? dim3(cgrid.x, cgrid.y, cgrid.z * kCheckZrun) : cgrid; }
 };
 
 // With one CTA per run a check of a small box is eight planes one after another on
@@ -105,6 +102,30 @@ inline void set_check_planes(Launch& L, int sms)
     const long long always = 1LL << 62;
     L.plane_runs = !env ? sms : (env[0] == '0' ? 0 : always);
     L.refine_plane_runs = !env ? 5LL * sms : L.plane_runs;
+}
+
+// Launches a check kernel on its runs: a CTA each, or (planes) a plane per CTA,
+// clusters of kCheckZrun making a run (zrun_terms).  The clusters are the launch's
+// and not the kernel's: kernels that declared clusters of one CTA took 3 to 8 us more
+// per check in the graphs' conditional bodies (mixed dual residual, a check each 10
+// sweeps, us per sweep: 64^3 9.4 -> 8.6, 32^3 6.7 -> 6.2).
+template <class... Params, class... Args>
+void launch_check(cudaStream_t st, const Launch& L, bool planes, void (*kern)(Params...), Args... args)
+{
+    if (!planes) {
+        kern<<<L.cgrid, L.block, 0, st>>>(args...);
+        return;
+    }
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim = {1, 1, kCheckZrun};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(L.cgrid.x, L.cgrid.y, L.cgrid.z * kCheckZrun);
+    cfg.blockDim = L.block;
+    cfg.stream = st;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);   // (an error is the capture's: capture_graph)
 }
 
 inline Launch make_launch(int lx, int ly, int lz, int bx, int by)
