@@ -1149,7 +1149,9 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
                 BCUDA(b, cudaEventSynchronize(b->ev[1]));
                 float ms = 0.f;
                 cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
-                if (ms / reps < best.sweep_ms) {
+                // (a clear win only: the checks' FP64 sums follow the list, and of two
+                // forms as fast as each other one run would take this, one that)
+                if (ms / reps < 0.995 * best.sweep_ms) {
                     best = t;
                     best.sweep_ms = ms / reps;
                 }
