@@ -42,14 +42,49 @@ def test_other_arrays_keep_their_allocator():
     assert names == ["default_allocator"]
 
 
-def test_memory_is_given_back():
-    def resident():
-        with open("/proc/self/statm") as f:
-            return int(f.read().split()[1]) * os.sysconf("SC_PAGE_SIZE")
+def mapped_mb():
+    with open("/proc/self/statm") as f:
+        return int(f.read().split()[0]) * os.sysconf("SC_PAGE_SIZE") / 1e6
 
-    L._host_array((HUGE // 8,)).fill(1.0)
+
+def test_freed_memory_is_kept_up_to_a_bound():
+    """Dropped arrays are found again, and no more of them than 512 MB is held."""
+    shape = (10 * HUGE // 8 - 3,)
+    a = L._host_array(shape)
+    at = a.ctypes.data
+    a.fill(2.0)
+    del a
+    b = L._host_array(shape)
+    assert b.ctypes.data == at          # the last one freed
+    b.fill(3.0)
+    del b
     gc.collect()
-    before = resident()
-    for _ in range(50):
-        L._host_array((10 * HUGE // 8 + 1,)).fill(1.0)
-    assert resident() - before < 64 << 20
+    before = mapped_mb()
+    many = [L._host_array((HUGE // 8 * k,)) for k in range(1, 60)]   # 3.5 GB, not touched
+    assert mapped_mb() - before > 3000
+    del many
+    gc.collect()
+    assert mapped_mb() - before < 600
+
+
+def test_allocation_from_several_threads():
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        held = []
+        for _ in range(60):
+            n = int(rng.integers(HUGE // 8, 4 * HUGE // 8))
+            a = L._host_array((n,))
+            a[0] = a[-1] = a[n // 2] = seed
+            held.append(a)
+            if len(held) > 5:
+                x = held.pop(int(rng.integers(len(held))))
+                assert x[0] == x[-1] == x[len(x) // 2] == seed
+        good.append(all(x[0] == x[-1] == seed for x in held))
+
+    good = []
+    threads = [threading.Thread(target=work, args=(i + 1,)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert good == [True] * 8
