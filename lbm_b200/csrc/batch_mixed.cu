@@ -1186,9 +1186,11 @@ lbm_status lbm_batch_tune(lbm_batch* b, lbm_batch_tuning* chosen)
     lbm_status ts = build_items(b);
     if (ts == LBM_OK) ts = time_graph(reps, [&] { singles(best, 0, reps); }, &best.sweep_ms);
     if (ts != LBM_OK) return ts;
-    // two sweeps per launch on z runs of 8, 16, 32 (per-sweep time = launch / 2)
-    // where that is worth the plan that a segment of passes starts with (some 3 us)
-    double least = 0.98 * best.sweep_ms;
+    // two sweeps per launch on z runs of 8, 16, 32 (per-sweep time = launch / 2).  With
+    // every box in its loop, as here, passes may be 4 % slower: once boxes have left,
+    // their list is rebuilt without them (ten of 33^3 12.95 us against 12.55, 8.26
+    // against 9.3 when they leave at different checks).
+    double least = 1.04 * best.sweep_ms;
     const int zr2[3] = {8, 16, 32};
     for (int zr : zr2) {
         lbm_batch_tuning t = best;
