@@ -247,7 +247,7 @@ def _dp(a: np.ndarray):
     return a.ctypes.data_as(C.POINTER(C.c_double))
 
 
-_HUGE_PAGE = 1 << 21
+_MAPPED_ARRAY = 1 << 17
 
 
 @functools.lru_cache(maxsize=None)
@@ -270,12 +270,13 @@ def _page_allocator():
 
 
 def _host_array(shape) -> np.ndarray:
-    """np.empty(shape) for a download, on huge pages where it holds some.  A
-    fresh array's pages are faulted in one by one by the copy into it, which
-    costs more than the copy (64 of 84 ms for sixty arrays of 2 to 4 MB); numpy
-    asks for huge pages from 4 MB on, and a plain allocation seldom holds one
-    of 2 MB whole, so the array starts on a huge page.  48 ms so."""
-    got = _page_allocator() if 8 * math.prod(shape) >= _HUGE_PAGE else None
+    """np.empty(shape) for a download, on memory of host_pages.cpp: huge pages
+    where it holds some, and pages of dropped arrays again.  A fresh array's
+    pages are faulted in one by one by the copy into it, which costs more than
+    the copy (64 of 84 ms for sixty arrays of 2 to 4 MB); numpy asks for huge
+    pages from 4 MB on, and a plain allocation seldom holds one of 2 MB whole.
+    48 ms on huge pages, 30 on pages of dropped arrays."""
+    got = _page_allocator() if 8 * math.prod(shape) >= _MAPPED_ARRAY else None
     if got is None:
         return np.empty(shape)
     set_handler, handler = got

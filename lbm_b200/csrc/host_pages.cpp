@@ -2,17 +2,18 @@
 //
 // A fresh array's pages are faulted in one by one by the copy into it, which
 // costs more than the copy itself.  NumPy takes the functions below as the
-// allocator of an array (its data memory handler, NEP 49), so the array owns its
-// memory as any other; one of a huge page or more starts on a huge page and is
-// faulted 2 MB at a time.
+// allocator of an array of 128 KB or more (its data memory handler, NEP 49), so the
+// array owns its memory as any other; one of a huge page or more starts on a huge
+// page and is faulted 2 MB at a time.
 //
 // A loop that downloads its results again and again drops the last ones when it
 // has the next.  Through malloc their memory goes back to the kernel or not by
 // what else lies at the heap's end, and the same run of ten boxes with sixty
 // downloads took 196 ms in one process and 231 in another.  So blocks are mapped
-// apart from the heap, and a few that were freed are kept for the next array of
-// their size: at most 512 MB and 256 blocks, their pages marked as free for the
-// kernel to take when it needs them (MADV_FREE).  Any thread may free or allocate;
+// apart from the heap, and those freed last are kept for the next array of their
+// size: of those on huge pages at most 512 MB, marked as free for the kernel to take
+// when it needs them (MADV_FREE), of smaller ones 64 MB (there the mark costs 40 us
+// an array, as much as the faults that it saves).  Any thread may free or allocate;
 // one that finds the list in use goes without.
 #include <sys/mman.h>
 
@@ -25,66 +26,96 @@
 namespace {
 
 constexpr size_t kHugePage = size_t(1) << 21, kPage = 4096;
-constexpr size_t kKeptBytes = size_t(512) << 20;
-constexpr int kKeptBlocks = 256;
+constexpr size_t kMapped = size_t(1) << 17, kGrain = size_t(1) << 16;   // smallest block mapped; sizes below a huge page
 
 // Ahead of every block.
 struct alignas(16) Header {
     size_t size;       // bytes asked for
-    size_t mapped;     // bytes of the block's huge pages, 0: from malloc
+    size_t mapped;     // bytes of the block's pages, 0: from malloc
 };
 
 Header* header_of(void* p) { return static_cast<Header*>(p) - 1; }
 
+void unmap_block(void* data, size_t mapped) { munmap(static_cast<char*>(data) - kPage, mapped + kPage); }
+
+// Freed blocks, the last one at the end.
 struct Kept {
-    void* data;
-    size_t mapped;
-};
-Kept g_kept[kKeptBlocks];
-int g_kept_count = 0;
-size_t g_kept_bytes = 0;
-std::mutex g_kept_mutex;
+    struct {
+        void* data;
+        size_t mapped;
+    } block[256];
+    int count = 0;
+    size_t bytes = 0;
+    const size_t most;
+    const bool give_back;   // mark the pages as free for the kernel
+    std::mutex mutex;
 
-// A kept block of exactly `mapped` bytes, the last one freed, or null.
-void* take_kept(size_t mapped)
-{
-    const std::unique_lock<std::mutex> lock(g_kept_mutex, std::try_to_lock);
-    if (!lock.owns_lock()) return nullptr;
-    for (int i = g_kept_count - 1; i >= 0; --i) {
-        if (g_kept[i].mapped != mapped) continue;
-        void* p = g_kept[i].data;
-        for (int k = i + 1; k < g_kept_count; ++k) g_kept[k - 1] = g_kept[k];
-        --g_kept_count;
-        g_kept_bytes -= mapped;
-        return p;
+    Kept(size_t limit, bool give) : most(limit), give_back(give) {}
+
+    // A block of exactly `mapped` bytes, the last one freed, or null.
+    void* take(size_t mapped)
+    {
+        const std::unique_lock<std::mutex> lock(mutex, std::try_to_lock);
+        if (!lock.owns_lock()) return nullptr;
+        for (int i = count - 1; i >= 0; --i) {
+            if (block[i].mapped != mapped) continue;
+            void* p = block[i].data;
+            drop(i, 1);
+            return p;
+        }
+        return nullptr;
     }
-    return nullptr;
-}
 
-bool keep(void* data, size_t mapped)
+    // Keeps a block, in the place of those kept longest where there is no room.
+    bool keep(void* data, size_t mapped)
+    {
+        if (mapped > most) return false;
+        const std::unique_lock<std::mutex> lock(mutex, std::try_to_lock);
+        if (!lock.owns_lock()) return false;
+        int out = 0;
+        for (size_t left = bytes; count - out == 256 || left + mapped > most; ++out) {
+            left -= block[out].mapped;
+            unmap_block(block[out].data, block[out].mapped);
+        }
+        drop(0, out);
+        if (give_back) madvise(data, mapped, MADV_FREE);
+        block[count].data = data;
+        block[count++].mapped = mapped;
+        bytes += mapped;
+        return true;
+    }
+
+private:
+    void drop(int at, int n)
+    {
+        for (int k = at; k < at + n; ++k) bytes -= block[k].mapped;
+        for (int k = at + n; k < count; ++k) block[k - n] = block[k];
+        count -= n;
+    }
+};
+
+// (never destroyed: arrays may be freed after the library's own end)
+Kept& kept_of(size_t size)
 {
-    const std::unique_lock<std::mutex> lock(g_kept_mutex, std::try_to_lock);
-    if (!lock.owns_lock() || g_kept_count == kKeptBlocks || mapped > kKeptBytes - g_kept_bytes) return false;
-    madvise(data, mapped, MADV_FREE);
-    g_kept[g_kept_count++] = {data, mapped};
-    g_kept_bytes += mapped;
-    return true;
+    static Kept* const huge = new Kept(size_t(512) << 20, true);
+    static Kept* const small = new Kept(size_t(64) << 20, false);
+    return size < kHugePage ? *small : *huge;
 }
 
-// Whole huge pages that start at the returned address, a page for the header
-// ahead of them.
+// `mapped` bytes from the returned address on, a huge page's where there is one,
+// and a page for the header ahead of them.
 void* map_block(size_t size, size_t mapped)
 {
-    const size_t room = mapped + kHugePage + kPage;
+    const size_t align = size < kHugePage ? kPage : kHugePage, room = mapped + align + kPage;
     char* base = static_cast<char*>(mmap(nullptr, room, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
     if (base == MAP_FAILED) return nullptr;
     const uintptr_t at = reinterpret_cast<uintptr_t>(base);
-    char* data = base + ((at + kPage + kHugePage - 1) / kHugePage * kHugePage - at);
+    char* data = base + ((at + kPage + align - 1) / align * align - at);
     const size_t ahead = static_cast<size_t>(data - kPage - base), behind = room - ahead - kPage - mapped;
     if (ahead) munmap(base, ahead);
     if (behind) munmap(data + mapped, behind);
     // (the last huge page where the array fills half of it; refused: ordinary pages)
-    madvise(data, (size + kHugePage / 2) / kHugePage * kHugePage, MADV_HUGEPAGE);
+    if (size >= kHugePage) madvise(data, (size + kHugePage / 2) / kHugePage * kHugePage, MADV_HUGEPAGE);
     return data;
 }
 
@@ -93,12 +124,13 @@ void* pages_malloc(void*, size_t size)
     if (size > SIZE_MAX / 2) return nullptr;
     void* data = nullptr;
     size_t mapped = 0;
-    if (size < kHugePage) {
+    if (size < kMapped) {
         Header* h = static_cast<Header*>(std::malloc(size + sizeof(Header)));
         data = h ? h + 1 : nullptr;
     } else {
-        mapped = (size + kHugePage - 1) / kHugePage * kHugePage;
-        data = take_kept(mapped);
+        const size_t grain = size < kHugePage ? kGrain : kHugePage;
+        mapped = (size + grain - 1) / grain * grain;
+        data = kept_of(size).take(mapped);
         if (!data) data = map_block(size, mapped);
     }
     if (data) *header_of(data) = {size, mapped};
@@ -116,9 +148,9 @@ void* pages_calloc(void* ctx, size_t n, size_t size)
 void pages_free(void*, void* p, size_t)
 {
     if (!p) return;
-    const size_t mapped = header_of(p)->mapped;
-    if (!mapped) std::free(header_of(p));
-    else if (!keep(p, mapped)) munmap(static_cast<char*>(p) - kPage, mapped + kPage);
+    const Header h = *header_of(p);
+    if (!h.mapped) std::free(header_of(p));
+    else if (!kept_of(h.size).keep(p, h.mapped)) unmap_block(p, h.mapped);
 }
 
 void* pages_realloc(void* ctx, void* p, size_t size)

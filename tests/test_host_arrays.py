@@ -20,7 +20,7 @@ def test_download_arrays_own_their_memory(shape):
     assert type(a) is np.ndarray and a.base is None
     assert (a.shape, a.dtype, a.strides) == (b.shape, b.dtype, b.strides)
     assert str(a.flags) == str(b.flags)
-    if a.nbytes >= HUGE:
+    if a.nbytes >= HUGE:   # (smaller ones start on a page)
         assert a.ctypes.data % HUGE == 0
     a[...] = 1.5
     assert pickle.loads(pickle.dumps(a)).sum() == a.sum()
@@ -65,6 +65,17 @@ def test_freed_memory_is_kept_up_to_a_bound():
     del many
     gc.collect()
     assert mapped_mb() - before < 600
+    # blocks of other sizes make room for those freed last
+    a = L._host_array(shape)
+    at = a.ctypes.data
+    del a
+    b = L._host_array(shape)
+    assert b.ctypes.data == at
+    small = [L._host_array((20000 + 100 * k,)) for k in range(400)]
+    at = small[-1].ctypes.data
+    while small:
+        small.pop(0)
+    assert L._host_array((20000 + 100 * 399,)).ctypes.data == at
 
 
 def test_allocation_from_several_threads():
